@@ -294,6 +294,35 @@ __host__ __device__ inline void philox_uniform8(uint64_t seed, uint32_t stream, 
   }
 }
 
+// Packed fp32 pairs (`.f32x2`, one instruction for two lanes of arithmetic) for loops bound by instruction issue.
+// Each op rounds exactly like its scalar form.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pk2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 pk2u(uint32_t lo, uint32_t hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // ---- CTA pairs (cta_group::2): one tcgen05.mma spans two CTAs of a cluster -------------------------
 // Each CTA stages its own 128 rows of A and its own half of B; the leader CTA (cluster rank 0)
 // issues the instruction and both CTAs receive their 128 accumulator rows in their own TMEM.

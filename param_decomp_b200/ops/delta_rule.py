@@ -1,7 +1,7 @@
 """Bindings of the gated-delta-rule and causal-conv kernels (`csrc/delta_rule.cu`).
 
-The recurrence runs in fp32 with the state on chip; the backward replays 64-token chunks from
-checkpointed states. Parity: param_decomp/target_ports/qwen3_5_moe.py:65-74,89-158.
+The recurrence runs in fp32 with the state on chip. The forward keeps each token's residual and the state at
+64-token chunk starts; the backward walks the state's cotangent once and forms the rest chunk by chunk. Parity: param_decomp/target_ports/qwen3_5_moe.py:65-74,89-158.
 """
 
 from __future__ import annotations
@@ -22,7 +22,7 @@ def _lib():
     lib = nv.lib()
     if not _configured:
         P, I = C.c_void_p, C.c_int
-        lib.pd_delta_rule_fwd.argtypes = [P] * 7 + [I] * 5 + [P]
+        lib.pd_delta_rule_fwd.argtypes = [P] * 8 + [I] * 5 + [P]
         lib.pd_delta_rule_bwd.argtypes = [P] * 13 + [I] * 5 + [P]
         lib.pd_conv1d_silu_fwd.argtypes = [P, P, P, I, I, I, I, P]
         lib.pd_conv1d_silu_bwd.argtypes = [P, P, P, P, P, I, I, I, I, P]
@@ -40,39 +40,46 @@ def conv_supported(x: Tensor, w: Tensor) -> bool:
             and nv.has_symbol("pd_conv1d_silu_fwd"))
 
 
+def _f32(t: Tensor) -> Tensor:
+    """Contiguous fp32 on a 16-byte boundary (the kernels copy 16 bytes at a time)."""
+    t = t.float().contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _DeltaRule(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor) -> Tensor:  # type: ignore[override]
-        q, k, v, g, beta = (t.float().contiguous() for t in (q, k, v, g, beta))
+        q, k, v, g, beta = (_f32(t) for t in (q, k, v, g, beta))
         B, T, H, dk = q.shape
         dv = v.shape[-1]
         o = torch.empty_like(v)
         need = any(ctx.needs_input_grad)
-        ckpt = torch.empty(B * H, (T + 63) // 64, dk, dv, device=q.device, dtype=torch.float32) if need else None
+        resid = torch.empty_like(v) if need else None
+        ckpt = torch.empty(B * H, (T + 63) // 64, dv, dk, device=q.device, dtype=torch.float32) if need else None
         rc = _lib().pd_delta_rule_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-                                      o.data_ptr(), ckpt.data_ptr() if need else None, B, T, H, dk, dv,
-                                      nv.current_stream_ptr())
+                                      o.data_ptr(), resid.data_ptr() if need else None,
+                                      ckpt.data_ptr() if need else None, B, T, H, dk, dv, nv.current_stream_ptr())
         nv.count_launch()
         if rc != 0:
             raise nv.NativeError(f"pd_delta_rule_fwd failed (code {rc})")
         if need:
-            ctx.save_for_backward(q, k, v, g, beta, ckpt)
+            ctx.save_for_backward(q, k, resid, g, beta, ckpt)
         return o
 
     @staticmethod
     def backward(ctx, d_o: Tensor):  # type: ignore[override]
-        q, k, v, g, beta, ckpt = ctx.saved_tensors
+        q, k, resid, g, beta, ckpt = ctx.saved_tensors
         B, T, H, dk = q.shape
-        dv = v.shape[-1]
-        d_o = d_o.float().contiguous()
-        dq, dk_, dv_ = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+        dv = resid.shape[-1]
+        d_o = _f32(d_o)
+        dq, dk_, dv_ = torch.empty_like(q), torch.empty_like(k), torch.empty_like(resid)
         dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
-        scratch = torch.empty(B * H, 64, dk, dv, device=q.device, dtype=torch.float32)
-        rc = _lib().pd_delta_rule_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-                                      d_o.data_ptr(), ckpt.data_ptr(), scratch.data_ptr(), dq.data_ptr(), dk_.data_ptr(),
+        gck = torch.empty_like(ckpt)
+        rc = _lib().pd_delta_rule_bwd(q.data_ptr(), k.data_ptr(), resid.data_ptr(), g.data_ptr(), beta.data_ptr(),
+                                      d_o.data_ptr(), ckpt.data_ptr(), gck.data_ptr(), dq.data_ptr(), dk_.data_ptr(),
                                       dv_.data_ptr(), dg.data_ptr(), dbeta.data_ptr(), B, T, H, dk, dv,
                                       nv.current_stream_ptr())
-        nv.count_launch()
+        nv.count_launch(2)
         if rc != 0:
             raise nv.NativeError(f"pd_delta_rule_bwd failed (code {rc})")
         return dq, dk_, dv_, dg, dbeta

@@ -902,3 +902,33 @@ def test_moe_fused_lazy_masks_match_eager(nv):
         assert rel(a[1][kk], b[1][kk]) < 5e-2, (kk, rel(a[1][kk], b[1][kk]))
     for kk in b[2]:
         assert rel(a[2][kk], b[2][kk]) < 5e-2, (kk, rel(a[2][kk], b[2][kk]))
+
+
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 128), (32, 32)])
+@pytest.mark.parametrize("T", [1, 16, 65, 191])
+def test_delta_rule_tiles_against_64_bits(nv, dk, dv, T):
+    """Ends of 16-token stages and 64-token chunks, strong and weak decay, beta 0 and 1, an unaligned value tensor.
+    fp32 sums of at most 128 terms over a decaying state: 2^-24 sqrt(128) = 7e-7, four times that is allowed."""
+    from param_decomp_b200.models import ports
+    from param_decomp_b200.ops import delta_rule
+
+    torch.manual_seed(T)
+    B, H = 2, 3
+    q = ports.l2norm(torch.randn(B, T, H, dk, device="cuda")) * dk**-0.5
+    k = ports.l2norm(torch.randn(B, T, H, dk, device="cuda"))
+    v = torch.empty(B * T * H * dv + 1, device="cuda")[1:].view(B, T, H, dv).normal_()
+    g = -torch.rand(B, T, H, device="cuda") * torch.tensor([0.02, 1.0, 8.0], device="cuda")
+    beta = torch.rand(B, T, H, device="cuda").round(decimals=1)
+    go = torch.randn_like(v)
+    ins = [t.detach().requires_grad_(True) for t in (q, k, v, g, beta)]
+    out = delta_rule.gated_delta_rule(*ins)
+    out.backward(go)
+    ref_ins = [t.detach().double().requires_grad_(True) for t in (q, k, v, g, beta)]
+    ref = ports._delta_rule_sequential(*ref_ins)
+    ref.backward(go.double())
+    _done(nv)
+    for name, a, b in zip("o q k v g beta".split(), [out] + [t.grad for t in ins], [ref] + [t.grad for t in ref_ins]):
+        err = float((a.double() - b).norm() / (b.norm() + 1e-9))
+        assert err < 3e-6, (name, err)
+    with torch.no_grad():  # the form without saved states gives the same values
+        assert torch.equal(delta_rule.gated_delta_rule(*ins), out)
