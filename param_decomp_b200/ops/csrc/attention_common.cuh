@@ -41,10 +41,10 @@ __device__ __forceinline__ void named_barrier_softmax() {
 }
 
 
-inline int encode_bthd(CUtensorMap* tm, const void* p, int B, int T, int heads, int hd) {
-  // [B, T, heads * hd] bf16 viewed as (inner = heads*hd, rows = T, batch = B); box = 64 columns x 128 rows
+inline int encode_bthd(CUtensorMap* tm, const void* p, int B, int T, int heads, int hd, int rows = kTile) {
+  // [B, T, heads * hd] bf16 viewed as (inner = heads*hd, rows = T, batch = B); box = 64 columns x `rows` rows
   return encode_tmap(tm, p, 2, false, static_cast<uint64_t>(heads) * hd, T, static_cast<uint64_t>(heads) * hd, B,
-                     static_cast<uint64_t>(T) * heads * hd, 64, kTile);
+                     static_cast<uint64_t>(T) * heads * hd, 64, rows);
 }
 
 inline bool bad_shape(int B, int T, int H, int Hkv, int hd) {

@@ -6,12 +6,18 @@
 // attention by head // (H / Hkv). The log-sum-exp is kept per (b, h, t) in base-2 units of the
 // scaled scores for the backward.
 //
-// Forward, one CTA per (128 query rows, head, batch); warps 0-3 = softmax (one query row per
-// thread = one TMEM lane), warp 4 = TMA producer, warp 5 = MMA issuer:
-//     S = Q K_j^T  (TMEM)  ->  online softmax in registers  ->  P_j (bf16, shared)  ->  O_j = P_j V_j (TMEM)
-// O_j is read back and accumulated in registers with the usual running-max correction, so nothing
-// in TMEM ever has to be rescaled. With hd = 64 a CTA takes 256 TMEM columns and 112 KB of shared
-// memory, so two CTAs share an SM and overlap each other's softmax and tensor phases.
+// Forward: CTAs walk the (128 query rows, head, batch) items, longest first, two CTAs to an SM; warps 0-3 = softmax
+// (one query row per thread = one TMEM lane), warp 4 = TMA producer, warp 5 = MMA issuer. Keys come 64 at a time:
+//     S = Q K_n^T  (TMEM, two buffers)  ->  online softmax in registers  ->  P_n (bf16, TMEM)  ->  O += P_n V_n (TMEM)
+// S of the next 64 keys is formed while the softmax warps work on the current ones, also across items, so they wait
+// neither for the tensor pipe nor for a new item's first loads. A row's scores are read once into registers; P goes
+// back to tensor memory over the scores it came from, as the A operand of P V, and never touches shared memory. O
+// stays in TMEM and is rescaled only when a row's maximum grows by more than 2^8 over the one its exponents refer to
+// (l, O and the final quotient share that reference, so the result is the same). Tiles off the diagonal of
+// unsegmented calls take no mask arithmetic. 256 TMEM columns and at most 98 KB a CTA; K and V halves share one ring in the
+// order the tensor pipe takes them. What bounds it is the exponentials (16 lanes a clock: 1024 cycles per 128 x 128).
+// B 64, T 512, 12 heads of 64: 152 us with one 128-key S at a time, P through shared memory and O in registers, 88 us
+// now; B 4, T 2048, 32 / 8 heads of 128: 440 -> 174 us (790 TFLOP/s). One item per CTA and 128 keys a step: 100, 215 us.
 //
 // Backward, one CTA per (128 key rows, kv head, batch), looping over the query heads of the group
 // and the query tiles that see this key tile:
@@ -48,65 +54,88 @@ struct AttnArgs {
   int* status;
 };
 
+constexpr int kSub = 64;  // keys per softmax step of the forward
+
 template <int HD>
 struct FwdPlan {
   static constexpr int kQBytes = kTile * HD * 2;
-  static constexpr int kKVBytes = kTile * HD * 2;
-  static constexpr int kPBytes = kTile * kTile * 2;
-  static constexpr int kStages = 2;                 // K ring
-  static constexpr int kVStages = HD == 64 ? 1 : 2;  // one V buffer keeps a CTA under half an SM's shared memory
-  static constexpr int kTotal = kQBytes + (kStages + kVStages) * kKVBytes + kPBytes + 1024 /*align*/ + 1024 /*barriers, seg ids*/;
-  static constexpr uint32_t kTmemCols = 256;  // S: 128 columns, O: HD columns at column 128
+  static constexpr int kSlotBytes = kSub * HD * 2;      // 64 rows of K or V
+  static constexpr int kSlots = HD == 64 ? 8 : 4;       // 64 KB: a CTA stays under half an SM's shared memory
+  static constexpr int kTotal = kQBytes + kSlots * kSlotBytes + 1024 /*align*/ + 256 /*barriers*/ + 4 * kSub * 4 /*segment ids*/;
+  static constexpr uint32_t kTmemCols = 256;            // S / P buffers [0, 64) and [64, 128), O [128, 128 + hd)
+};
+constexpr float kRescaleLog2 = 8.0f;
+
+// The 64-key steps of the items a CTA walks (w, w + stride, ...), in order.
+struct StepCursor {
+  const AttnArgs& a;
+  int w, stride, items, n_qt;
+  int j = 0, n_sub = 0, qt = 0, h = 0, b = 0;
+  __device__ StepCursor(const AttnArgs& args, int first, int step) : a(args), w(first), stride(step) {
+    n_qt = a.T / kTile;
+    items = n_qt * a.H * a.B;
+    open();
+  }
+  __device__ bool done() const { return w >= items; }
+  __device__ bool last() const { return j + 1 == n_sub; }
+  __device__ void open() {  // longest items first; neighbours share K and V of a (batch, kv head)
+    if (done()) return;
+    const int hb = w % (a.H * a.B);
+    qt = n_qt - 1 - w / (a.H * a.B);
+    h = hb % a.H;
+    b = hb / a.H;
+    n_sub = (kTile / kSub) * (a.causal ? qt + 1 : n_qt);
+  }
+  __device__ void advance() {
+    if (++j == n_sub) {
+      j = 0;
+      w += stride;
+      open();
+    }
+  }
 };
 
 // ------------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------------
 template <int HD>
-__global__ void __launch_bounds__(kFwdThreads, HD == 64 ? 2 : 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
-                                                                const __grid_constant__ CUtensorMap tmK,
-                                                                const __grid_constant__ CUtensorMap tmV,
-                                                                const AttnArgs args) {
+__global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
+                                                                  const __grid_constant__ CUtensorMap tmK,
+                                                                  const __grid_constant__ CUtensorMap tmV,
+                                                                  const AttnArgs args) {
   using Plan = FwdPlan<HD>;
-  constexpr int kStages = Plan::kStages;
-  constexpr int kVStages = Plan::kVStages;
+  constexpr int kSlots = Plan::kSlots;
   constexpr int kKB = HD / 64;  // 64-wide K blocks of the head dimension
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sm_q = base;
-  const uint32_t sm_k = sm_q + Plan::kQBytes;
-  const uint32_t sm_v = sm_k + kStages * Plan::kKVBytes;
-  const uint32_t sm_p = sm_v + kVStages * Plan::kKVBytes;
-  const uint32_t sm_bar = sm_p + Plan::kPBytes;
-  // barriers: q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, p_full, o_full
-  const uint32_t bar_q = sm_bar;
-  const uint32_t bar_kf = bar_q + 8, bar_ke = bar_kf + 16, bar_vf = bar_ke + 16, bar_ve = bar_vf + 16;
-  const uint32_t bar_s = bar_ve + 16, bar_p = bar_s + 8, bar_o = bar_p + 8;
-  const uint32_t tmem_slot = bar_o + 8;
+  const uint32_t sm_kv = sm_q + Plan::kQBytes;
+  const uint32_t sm_bar = sm_kv + kSlots * Plan::kSlotBytes;
+  // barriers: q_full, q_empty, slot_full[8], slot_empty[8], s_full[2], p_full[2], o_full, o_empty
+  const uint32_t bar_qf = sm_bar, bar_qe = bar_qf + 8;
+  const uint32_t bar_f = bar_qe + 8, bar_e = bar_f + 64, bar_s = bar_e + 64, bar_p = bar_s + 16;
+  const uint32_t bar_o = bar_p + 16, bar_oe = bar_o + 8;
+  const uint32_t tmem_slot = bar_oe + 8;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + (tmem_slot + 4 - base));
-  int* seg_k = reinterpret_cast<int*>(gbase + (sm_bar + 256 - base));  // [128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heavy (late) query tiles first so the causal triangle packs well
-  const int n_qt = args.T / kTile;
-  const int qt = n_qt - 1 - static_cast<int>(blockIdx.x);
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hk = h / (args.H / args.Hkv);
-  const int n_kv = args.causal ? qt + 1 : n_qt;
+  int* seg_k = reinterpret_cast<int*>(gbase + (sm_bar + 256 - base)) + (warp & 3) * kSub;  // a softmax warp's ids
 
   if (threadIdx.x == 0) {
-    mbar_init(bar_q, 1);
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(bar_kf + 8 * s, 1);
-      mbar_init(bar_ke + 8 * s, 1);
-      mbar_init(bar_vf + 8 * s, 1);
-      mbar_init(bar_ve + 8 * s, 1);
+    mbar_init(bar_qf, 1);
+    mbar_init(bar_qe, 1);
+    for (int i = 0; i < kSlots; ++i) {
+      mbar_init(bar_f + 8 * i, 1);
+      mbar_init(bar_e + 8 * i, 1);
     }
-    mbar_init(bar_s, 1);
-    mbar_init(bar_p, kSoftmaxThreads);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_s + 8 * i, 1);
+      mbar_init(bar_p + 8 * i, kSoftmaxThreads);
+    }
     mbar_init(bar_o, 1);
+    mbar_init(bar_oe, kSoftmaxThreads);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -121,196 +150,249 @@ __global__ void __launch_bounds__(kFwdThreads, HD == 64 ? 2 : 1) attn_fwd_kernel
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_s = *tmem_slot_ptr;
-  const uint32_t tmem_o = tmem_s + 128;
+  const uint32_t tmem_o = tmem_s + 2 * kSub;
+  const int w0 = static_cast<int>(blockIdx.x), wstep = static_cast<int>(gridDim.x);
 
+  // Producer and MMA issuer walk one sequence of tensor steps: S_0, S_1, then P V_n, S_{n+2} for every n. Each step
+  // takes the next slot of the ring (64 rows of K for S, of V for P V).
   if (warp == 4) {
     // ---------------- TMA producer (whole warp walks the loop, one elected lane issues) ----------------
-    if (elect_one_sync()) {
-      mbar_expect_tx(bar_q, Plan::kQBytes);
-      for (int c = 0; c < kKB; ++c) tma_load_3d(sm_q + c * (kTile * 128), &tmQ, bar_q, h * HD + 64 * c, qt * kTile, b);
-    }
-    for (int j = 0; j < n_kv; ++j) {
-      const int st = j % kStages;
-      const uint32_t ph = static_cast<uint32_t>((j / kStages) & 1);
-      if (!mbar_wait_warp(bar_ke + 8 * st, ph ^ 1, abort_flag)) {
-        if (lane == 0) atomicCAS(args.status, 0, kTimeoutProducer);
-        break;
-      }
+    StepCursor sc(args, w0, wstep), vc(args, w0, wstep);
+    uint32_t slot = 0, phase = 0, q_count = 0;
+    bool ok = true;
+    auto load = [&](const StepCursor& c, const CUtensorMap* tm) {
+      ok = mbar_wait_warp(bar_e + 8 * slot, phase ^ 1, abort_flag);
+      if (!ok) return;
       if (elect_one_sync()) {
-        mbar_expect_tx(bar_kf + 8 * st, Plan::kKVBytes);
-        for (int c = 0; c < kKB; ++c)
-          tma_load_3d(sm_k + st * Plan::kKVBytes + c * (kTile * 128), &tmK, bar_kf + 8 * st, hk * HD + 64 * c,
-                      j * kTile, b);
+        mbar_expect_tx(bar_f + 8 * slot, Plan::kSlotBytes);
+        const int hk = c.h / (args.H / args.Hkv);
+        for (int i = 0; i < kKB; ++i)
+          tma_load_3d(sm_kv + slot * Plan::kSlotBytes + i * (kSub * 128), tm, bar_f + 8 * slot, hk * HD + 64 * i,
+                      c.j * kSub, c.b);
       }
-      const int vs = j % kVStages;
-      const uint32_t vph = static_cast<uint32_t>((j / kVStages) & 1);
-      if (!mbar_wait_warp(bar_ve + 8 * vs, vph ^ 1, abort_flag)) {
-        if (lane == 0) atomicCAS(args.status, 0, kTimeoutProducer);
-        break;
+      if (++slot == kSlots) {
+        slot = 0;
+        phase ^= 1;
       }
-      if (elect_one_sync()) {
-        mbar_expect_tx(bar_vf + 8 * vs, Plan::kKVBytes);
-        for (int c = 0; c < kKB; ++c)
-          tma_load_3d(sm_v + vs * Plan::kKVBytes + c * (kTile * 128), &tmV, bar_vf + 8 * vs, hk * HD + 64 * c,
-                      j * kTile, b);
+    };
+    auto next_k = [&]() {
+      if (sc.done()) return;
+      if (sc.j == 0) {  // a new item: its queries, once the last S of the item before has been formed
+        ok = mbar_wait_warp(bar_qe, (q_count & 1) ^ 1, abort_flag);
+        if (!ok) return;
+        ++q_count;
+        if (elect_one_sync()) {
+          mbar_expect_tx(bar_qf, Plan::kQBytes);
+          for (int i = 0; i < kKB; ++i) tma_load_3d(sm_q + i * (kTile * 128), &tmQ, bar_qf, sc.h * HD + 64 * i, sc.qt * kTile, sc.b);
+        }
       }
+      load(sc, &tmK);
+      sc.advance();
+    };
+    next_k();
+    if (ok) next_k();
+    while (ok && !vc.done()) {
+      load(vc, &tmV);
+      vc.advance();
+      if (ok) next_k();
     }
+    if (!ok && lane == 0) atomicCAS(args.status, 0, kTimeoutProducer);
   } else if (warp == 5) {
     // ---------------- MMA issuer (whole warp walks the loop, one elected lane issues) ----------------
-    {
-      constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);
-      constexpr uint32_t idesc_o = make_idesc_bf16(kTile, HD, 0, 1);
-      bool ok = mbar_wait_warp(bar_q, 0, abort_flag);
-      auto issue_s = [&](int j) {
-        const int st = j % kStages;
-        if (!mbar_wait_warp(bar_kf + 8 * st, static_cast<uint32_t>((j / kStages) & 1), abort_flag)) return false;
-        tc_fence_after();
-        if (elect_one_sync()) {
-#pragma unroll
-          for (int c = 0; c < kKB; ++c) {
-            const uint64_t ad = make_smem_desc(sm_q + c * (kTile * 128), 16, 1024);
-            const uint64_t bd = make_smem_desc(sm_k + st * Plan::kKVBytes + c * (kTile * 128), 16, 1024);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) umma_bf16(tmem_s, ad + k * 2, bd + k * 2, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
-          }
-          umma_commit(bar_ke + 8 * st);
-          umma_commit(bar_s);
-        }
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        // P_j is in shared memory; the softmax warps are also done with S_j and O_{j-1}
-        if (!mbar_wait_warp(bar_p, static_cast<uint32_t>(j & 1), abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        if (j + 1 < n_kv && !issue_s(j + 1)) { ok = false; break; }
-        const int vs = j % kVStages;
-        if (!mbar_wait_warp(bar_vf + 8 * vs, static_cast<uint32_t>((j / kVStages) & 1), abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one_sync()) {
-          const uint64_t vd = make_smem_desc(sm_v + vs * Plan::kKVBytes, kTile * 128, 1024);
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {  // two 64-wide blocks of the key index
-            const uint64_t pd_ = make_smem_desc(sm_p + c * (kTile * 128), 16, 1024);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16(tmem_o, pd_ + k * 2, vd + (c * 4 + k) * (2048 >> 4), idesc_o, (c > 0 || k > 0) ? 1u : 0u);
-          }
-          umma_commit(bar_ve + 8 * vs);
-          umma_commit(bar_o);
-        }
+    constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kSub, 0, 0);
+    constexpr uint32_t idesc_o = make_idesc_bf16(kTile, HD, 0, 1);
+    StepCursor sc(args, w0, wstep), vc(args, w0, wstep);
+    uint32_t slot = 0, phase = 0, q_count = 0, s_count = 0, v_count = 0, o_count = 0;
+    bool ok = true;
+    auto advance_slot = [&]() {
+      if (++slot == kSlots) {
+        slot = 0;
+        phase ^= 1;
       }
-      if (!ok && lane == 0) atomicCAS(args.status, 0, kTimeoutMma);
+    };
+    auto next_s = [&]() {
+      if (sc.done()) return;
+      if (sc.j == 0) {
+        ok = mbar_wait_warp(bar_qf, q_count & 1, abort_flag);
+        ++q_count;
+      }
+      if (ok) ok = mbar_wait_warp(bar_f + 8 * slot, phase, abort_flag);
+      if (!ok) return;
+      tc_fence_after();
+      if (elect_one_sync()) {
+        const uint32_t d = tmem_s + (s_count & 1) * kSub;
+#pragma unroll
+        for (int c = 0; c < kKB; ++c) {
+          const uint64_t ad = make_smem_desc(sm_q + c * (kTile * 128), 16, 1024);
+          const uint64_t bd = make_smem_desc(sm_kv + slot * Plan::kSlotBytes + c * (kSub * 128), 16, 1024);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_bf16(d, ad + k * 2, bd + k * 2, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(bar_e + 8 * slot);
+        umma_commit(bar_s + 8 * (s_count & 1));
+        if (sc.last()) umma_commit(bar_qe);
+      }
+      ++s_count;
+      advance_slot();
+      sc.advance();
+    };
+    next_s();
+    if (ok) next_s();
+    while (ok && !vc.done()) {
+      // P_n is in tensor memory; the softmax warps are done with S_n and with rescaling O
+      const uint32_t buf = v_count & 1;
+      ok = mbar_wait_warp(bar_p + 8 * buf, (v_count >> 1) & 1, abort_flag) &&
+           mbar_wait_warp(bar_f + 8 * slot, phase, abort_flag);
+      if (ok && vc.j == 0) {  // O of the item before has been read out
+        ok = mbar_wait_warp(bar_oe, (o_count & 1) ^ 1, abort_flag);
+        ++o_count;
+      }
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one_sync()) {
+        const uint64_t vd = make_smem_desc(sm_kv + slot * Plan::kSlotBytes, kSub * 128, 1024);
+#pragma unroll
+        for (int k = 0; k < kSub / 16; ++k)  // 16 keys: eight columns of P, two 8-row groups of V
+          umma_bf16_ts(tmem_o, tmem_s + buf * kSub + 8 * k, vd + k * (2048 >> 4), idesc_o, (vc.j > 0 || k > 0) ? 1u : 0u);
+        umma_commit(bar_e + 8 * slot);
+        umma_commit(bar_o);
+      }
+      advance_slot();
+      vc.advance();
+      if (!sc.done()) {  // S_{n+2} overwrites P_n: P V_n has read it
+        ok = mbar_wait_warp(bar_o, v_count & 1, abort_flag);
+        if (ok) next_s();
+      }
+      ++v_count;
     }
+    if (!ok && lane == 0) atomicCAS(args.status, 0, kTimeoutMma);
   } else {
     // ---------------- softmax + output (one query row per thread) ----------------
     const int row = threadIdx.x;  // 0..127 = TMEM lane
-    const int q_idx = qt * kTile + row;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    const int seg_q = args.segment_ids ? args.segment_ids[b * args.T + q_idx] : 0;
-    float m_run = -INFINITY, l_run = 0.0f;
-    float o[HD];
-#pragma unroll
-    for (int i = 0; i < HD; ++i) o[i] = 0.0f;
+    const f32x2 scale2 = pk2(args.scale_log2, args.scale_log2);
+    uint32_t n = 0;  // steps so far: S buffer n & 1
     bool ok = true;
-    for (int j = 0; j < n_kv && ok; ++j) {
-      if (args.segment_ids) {
-        named_barrier_softmax();  // everyone is done with the previous tile's ids
-        seg_k[row] = args.segment_ids[b * args.T + j * kTile + row];
-        named_barrier_softmax();
-      }
-      if (!mbar_wait(bar_s, static_cast<uint32_t>(j & 1), abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      const bool diag = args.causal && j == qt;
-      // pass 1: row maximum of the scaled, masked scores
-      float m_new = m_run;
-      uint32_t r[32];
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        tmem_ld_32x32(tmem_s + lane_base + c * 32, r);
-        tmem_ld_wait();
+    StepCursor sc(args, w0, wstep);
+    while (ok && !sc.done()) {
+      const int q_idx = sc.qt * kTile + row;
+      const int* seg_row = args.segment_ids ? args.segment_ids + static_cast<long long>(sc.b) * args.T : nullptr;
+      const int seg_q = seg_row ? seg_row[q_idx] : 0;
+      float m_ref = -INFINITY;  // the maximum the exponents of l and O refer to
+      f32x2 l2 = 0ull;
+      const int diag_j = args.causal ? sc.qt * (kTile / kSub) : 0x7FFFFFFF;  // steps from here on cross the diagonal
+      for (int j = 0; j < sc.n_sub; ++j, ++n) {
+        if (seg_row) {  // the warp's own copy of the step's ids
+          __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int col = c * 32 + i;
-          const bool keep = (!diag || col <= row) && (!args.segment_ids || seg_k[col] == seg_q);
-          if (keep) m_new = fmaxf(m_new, __uint_as_float(r[i]) * args.scale_log2);
+          for (int c = 0; c < kSub / 32; ++c) seg_k[c * 32 + lane] = seg_row[j * kSub + c * 32 + lane];
+          __syncwarp();
         }
-      }
-      // O_{j-1} (computed against the previous maximum) joins the register accumulator first
-      if (j > 0) {
-        if (!mbar_wait(bar_o, static_cast<uint32_t>((j - 1) & 1), abort_flag)) { ok = false; break; }
+        const uint32_t buf = n & 1;
+        if (!mbar_wait_warp(bar_s + 8 * buf, (n >> 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
+        const uint32_t tmem_sp = tmem_s + buf * kSub + lane_base;
+        uint32_t r[2][32];
 #pragma unroll
-        for (int c = 0; c < HD / 32; ++c) {
-          tmem_ld_32x32(tmem_o + lane_base + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[c * 32 + i] += __uint_as_float(r[i]);
-        }
-      }
-      const float alpha = (m_run == -INFINITY) ? 0.0f : fast_exp2(m_run - m_new);
-      l_run *= alpha;
-#pragma unroll
-      for (int i = 0; i < HD; ++i) o[i] *= alpha;
-      m_run = m_new;
-      // pass 2: probabilities -> shared memory (bf16, swizzled K-major blocks of 64 keys)
-      float l_add = 0.0f;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        tmem_ld_32x32(tmem_s + lane_base + c * 32, r);
+        for (int c = 0; c < 2; ++c) tmem_ld_32x32(tmem_sp + c * 32, r[c]);
         tmem_ld_wait();
-        uint32_t packed[16];
+        constexpr uint32_t kNegInf = 0xFF800000u;
+        if (j >= diag_j) {
+          const int lim = row - (j - diag_j) * kSub;  // last key column this row sees
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p2[2];
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int col = c * 32 + i + e;
-            const bool keep = (!diag || col <= row) && (!args.segment_ids || seg_k[col] == seg_q);
-            p2[e] = keep ? fast_exp2(__uint_as_float(r[i + e]) * args.scale_log2 - m_new) : 0.0f;
-          }
-          packed[i >> 1] = pack_bf16(p2[0], p2[1]);
-          // the sum uses the rounded values the tensor core will see
-          const __nv_bfloat162 hb = *reinterpret_cast<__nv_bfloat162*>(&packed[i >> 1]);
-          const float2 f = __bfloat1622float2(hb);
-          l_add += f.x + f.y;
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i > lim) r[c][i] = kNegInf;
         }
-        const uint32_t blk = sm_p + (c >> 1) * (kTile * 128);
+        if (seg_row) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const int4 id = *reinterpret_cast<const int4*>(seg_k + c * 32 + i);
+              if (id.x != seg_q) r[c][i] = kNegInf;
+              if (id.y != seg_q) r[c][i + 1] = kNegInf;
+              if (id.z != seg_q) r[c][i + 2] = kNegInf;
+              if (id.w != seg_q) r[c][i + 3] = kNegInf;
+            }
+        }
+        float mx[4];  // four chains of the row maximum (the scale is positive)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mx[c] = __uint_as_float(r[c >> 1][(c & 1) * 16]);
+#pragma unroll
+        for (int i = 1; i < 16; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mx[c] = fmaxf(mx[c], __uint_as_float(r[c >> 1][(c & 1) * 16 + i]));
+        const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * args.scale_log2;
+        const bool grow = j == 0 ? m_tile > -INFINITY : m_tile > m_ref + kRescaleLog2;
+        if (j == 0) {
+          if (grow) m_ref = m_tile;
+        } else if (__any_sync(0xffffffffu, grow)) {
+          const float alpha = grow ? fast_exp2(m_ref - m_tile) : 1.0f;  // 0 where nothing was seen before
+          if (grow) m_ref = m_tile;
+          l2 = mul2(l2, pk2(alpha, alpha));
+          if (!mbar_wait_warp(bar_o, (n - 1) & 1, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < HD / 16; ++c) {
+            uint32_t o[16];
+            tmem_ld_16(tmem_o + lane_base + c * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_16(tmem_o + lane_base + c * 16, o);
+          }
+        }
+        const float m_sub = m_ref == -INFINITY ? 0.0f : -m_ref;  // a row with nothing kept yet: exp2(-inf) = 0
+        const f32x2 m2 = pk2(m_sub, m_sub);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t packed[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float2 x = unpack2(fma2(pk2u(r[c][2 * i], r[c][2 * i + 1]), scale2, m2));
+            packed[i] = pack_bf16(fast_exp2(x.x), fast_exp2(x.y));
+            l2 = add2(l2, unpack_bf16_2(packed[i]));  // the sum uses the rounded values the tensor core will see
+          }
+          tmem_st_16(tmem_sp + c * 16, packed);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(bar_p + 8 * buf);
+      }
+      if (!ok) break;
+      // both of the last two P V may still run, and a parity only tells neighbouring phases apart: wait for each
+      if (!mbar_wait_warp(bar_o, (n - 2) & 1, abort_flag) || !mbar_wait_warp(bar_o, (n - 1) & 1, abort_flag)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const float2 lp = unpack2(l2);
+      const float l_run = lp.x + lp.y;
+      const float inv = 1.0f / l_run;
+      __nv_bfloat16* dst = args.out + ((static_cast<long long>(sc.b) * args.T + q_idx) * args.H + sc.h) * HD;
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(tmem_o + lane_base + c * 32, o);
+        tmem_ld_wait();
+        if (c == HD / 32 - 1) {  // the tensor pipe may start on the next item's O
+          tc_fence_before();
+          mbar_arrive(bar_oe);
+        }
+        float f[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * inv;
 #pragma unroll
         for (int g = 0; g < 4; ++g)
-          st_shared_v4(blk + swz(row, (c & 1) * 4 + g),
-                       make_uint4(packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]));
+          *reinterpret_cast<uint4*>(dst + c * 32 + 8 * g) =
+              make_uint4(pack_bf16(f[8 * g], f[8 * g + 1]), pack_bf16(f[8 * g + 2], f[8 * g + 3]),
+                         pack_bf16(f[8 * g + 4], f[8 * g + 5]), pack_bf16(f[8 * g + 6], f[8 * g + 7]));
       }
-      l_run += l_add;
-      tc_fence_before();
-      fence_proxy_async_smem();
-      mbar_arrive(bar_p);
-    }
-    if (ok && n_kv > 0) {
-      if (!mbar_wait(bar_o, static_cast<uint32_t>((n_kv - 1) & 1), abort_flag)) ok = false;
-      if (ok) {
-        tc_fence_after();
-        uint32_t r[32];
-#pragma unroll
-        for (int c = 0; c < HD / 32; ++c) {
-          tmem_ld_32x32(tmem_o + lane_base + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[c * 32 + i] += __uint_as_float(r[i]);
-        }
-        const float inv = 1.0f / l_run;
-        __nv_bfloat16* dst = args.out + ((static_cast<long long>(b) * args.T + q_idx) * args.H + h) * HD;
-#pragma unroll
-        for (int g = 0; g < HD / 8; ++g) {
-          uint4 v;
-          v.x = pack_bf16(o[8 * g] * inv, o[8 * g + 1] * inv);
-          v.y = pack_bf16(o[8 * g + 2] * inv, o[8 * g + 3] * inv);
-          v.z = pack_bf16(o[8 * g + 4] * inv, o[8 * g + 5] * inv);
-          v.w = pack_bf16(o[8 * g + 6] * inv, o[8 * g + 7] * inv);
-          *reinterpret_cast<uint4*>(dst + 8 * g) = v;
-        }
-        if (args.lse) args.lse[(static_cast<long long>(b) * args.H + h) * args.T + q_idx] = m_run + log2f(l_run);
-      }
+      if (args.lse) args.lse[(static_cast<long long>(sc.b) * args.H + sc.h) * args.T + q_idx] = m_ref + log2f(l_run);
+      sc.j = sc.n_sub - 1;
+      sc.advance();
     }
     if (!ok) atomicCAS(args.status, 0, kTimeoutEpilogue);
   }
@@ -633,8 +715,9 @@ int launch_fwd(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
       return 300;
     configured = true;
   }
-  dim3 grid(a.T / kTile, a.H, a.B);
-  kern<<<grid, kFwdThreads, FwdPlan<HD>::kTotal, st>>>(q, k, v, a);
+  const long long items = static_cast<long long>(a.T / kTile) * a.H * a.B;
+  if (items > 0x3FFFFFFF) return kBadArgument;
+  kern<<<static_cast<unsigned>(std::min<long long>(items, 2 * 148)), kFwdThreads, FwdPlan<HD>::kTotal, st>>>(q, k, v, a);
   return cudaGetLastError() == cudaSuccess ? 0 : 400;
 }
 
@@ -662,8 +745,8 @@ extern "C" int pd_flash_attention_fwd(const void* q, const void* k, const void* 
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = encode_bthd(&tq, q, B, T, H, hd)) != 0) return 1000 + rc;
-  if ((rc = encode_bthd(&tk, k, B, T, Hkv, hd)) != 0) return 1000 + rc;
-  if ((rc = encode_bthd(&tv, v, B, T, Hkv, hd)) != 0) return 1000 + rc;
+  if ((rc = encode_bthd(&tk, k, B, T, Hkv, hd, kSub)) != 0) return 1000 + rc;
+  if ((rc = encode_bthd(&tv, v, B, T, Hkv, hd, kSub)) != 0) return 1000 + rc;
   AttnArgs a{};
   a.B = B; a.T = T; a.H = H; a.Hkv = Hkv; a.causal = causal;
   a.scale = 1.0f / sqrtf(static_cast<float>(hd));

@@ -166,13 +166,6 @@ __device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
   }
 }
 
-__device__ __forceinline__ uint32_t pack_bf16_2(f32x2 v) {  // (lo, hi) -> bf16x2 with lo in the low half
-  uint32_t r;
-  asm("{\n\t.reg .f32 lo, hi;\n\tmov.b64 {lo, hi}, %1;\n\tcvt.rn.bf16x2.f32 %0, hi, lo;\n\t}" : "=r"(r) : "l"(v));
-  return r;
-}
-// bf16x2 word -> the two values as an fp32 pair
-__device__ __forceinline__ f32x2 unpack_bf16_2(uint32_t w) { return pk2u(w << 16, w & 0xFFFF0000u); }
 // One Philox word -> its two 16-bit uniforms (b + 0.5) / 65536 as an fp32 pair: the bits go to the top of the
 // mantissa of a float in [1, 2), and 2^-17 - 1 (exact in fp32) is added - the same values as `bits16_to_unit`.
 __device__ __forceinline__ f32x2 philox_word_to_unit2(uint32_t w) {

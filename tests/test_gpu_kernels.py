@@ -932,3 +932,22 @@ def test_delta_rule_tiles_against_64_bits(nv, dk, dv, T):
         assert err < 3e-6, (name, err)
     with torch.no_grad():  # the form without saved states gives the same values
         assert torch.equal(delta_rule.gated_delta_rule(*ins), out)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("T,H,Hkv,B", [(128, 2, 1, 1), (256, 3, 3, 2), (640, 12, 4, 30)])
+def test_flash_attention_walks_items(nv, hd, T, H, Hkv, B):
+    """Fewer items than CTAs, and several items per CTA (1,800 at the largest) with growing maxima (late keys score
+    far above early ones, so O is rescaled) against fp32 softmax."""
+    from param_decomp_b200.models import ports
+    from param_decomp_b200.ops import attention as attn
+
+    torch.manual_seed(T)
+    q, k, v = (torch.randn(B, T, h, hd, device="cuda") for h in (H, Hkv, Hkv))
+    k = k * torch.linspace(0.5, 4.0, T, device="cuda")[None, :, None, None]
+    q, k, v = q.to(bf), k.to(bf), v.to(bf)
+    for causal in (True, False):
+        out = attn.flash_attention(q, k, v, causal)
+        ref = ports.sdpa_reference(q.float(), k.float(), v.float(), causal, None)
+        _done(nv)
+        assert rel(out, ref) < 6e-3, (causal, rel(out, ref))  # bf16 probabilities and outputs: 2^-8 each
