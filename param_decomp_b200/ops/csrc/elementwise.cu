@@ -639,81 +639,6 @@ __global__ void ci_squash_activity_jobs_bwd_kernel(const __nv_bfloat16* __restri
   }
 }
 
-// ---- vocabulary KL: one block per position ------------------------------------------------------
-// kl[row] = KL(softmax(lc[row]) || softmax(lm[row]));  dlm[row] = softmax(lm) - softmax(lc)
-// (the caller scales by the upstream gradient / number of positions inside the next GEMM).
-// Rows are `ld` elements apart (padded to a multiple of 8); V valid columns.
-__global__ void vocab_kl_kernel(const __nv_bfloat16* __restrict__ lc, const __nv_bfloat16* __restrict__ lm,
-                                __nv_bfloat16* __restrict__ dlm, float* __restrict__ kl, int V, long long ld) {
-  const long long row = blockIdx.x;
-  const __nv_bfloat16* a = lc + row * ld;
-  const __nv_bfloat16* b = lm + row * ld;
-  __shared__ float red[4][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // pass 1: row maxima
-  float ma = -INFINITY, mb = -INFINITY;
-  for (int i = threadIdx.x * 8; i < V; i += blockDim.x * 8) {
-    const uint4 qa = *reinterpret_cast<const uint4*>(a + i), qb = *reinterpret_cast<const uint4*>(b + i);
-    const __nv_bfloat16* ha = reinterpret_cast<const __nv_bfloat16*>(&qa);
-    const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&qb);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (i + k < V) { ma = fmaxf(ma, __bfloat162float(ha[k])); mb = fmaxf(mb, __bfloat162float(hb[k])); }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ma = fmaxf(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-    mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-  }
-  if (lane == 0) { red[0][warp] = ma; red[1][warp] = mb; }
-  __syncthreads();
-  ma = red[0][0]; mb = red[1][0];
-  for (int w = 1; w < nw; ++w) { ma = fmaxf(ma, red[0][w]); mb = fmaxf(mb, red[1][w]); }
-  __syncthreads();
-  // pass 2: partition functions and the cross term sum exp(a - ma) * (a - b)
-  float sa = 0.f, sb = 0.f, cross = 0.f;
-  for (int i = threadIdx.x * 8; i < V; i += blockDim.x * 8) {
-    const uint4 qa = *reinterpret_cast<const uint4*>(a + i), qb = *reinterpret_cast<const uint4*>(b + i);
-    const __nv_bfloat16* ha = reinterpret_cast<const __nv_bfloat16*>(&qa);
-    const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&qb);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (i + k < V) {
-        const float x = __bfloat162float(ha[k]), y = __bfloat162float(hb[k]);
-        const float ea = __expf(x - ma);
-        sa += ea; sb += __expf(y - mb); cross += ea * (x - y);
-      }
-    }
-  }
-  sa = warp_sum(sa); sb = warp_sum(sb); cross = warp_sum(cross);
-  if (lane == 0) { red[0][warp] = sa; red[1][warp] = sb; red[2][warp] = cross; }
-  __syncthreads();
-  sa = 0.f; sb = 0.f; cross = 0.f;
-  for (int w = 0; w < nw; ++w) { sa += red[0][w]; sb += red[1][w]; cross += red[2][w]; }
-  const float lsa = ma + __logf(sa), lsb = mb + __logf(sb);
-  // KL = sum p_a (a - lsa - b + lsb) = cross / sa - lsa + lsb
-  if (threadIdx.x == 0) kl[row] = cross / sa - lsa + lsb;
-  // pass 3: gradient wrt the masked logits
-  if (dlm != nullptr) {
-    __nv_bfloat16* d = dlm + row * ld;
-    const float ia = 1.f / sa, ib = 1.f / sb;
-    for (int i = threadIdx.x * 8; i < V; i += blockDim.x * 8) {
-      const uint4 qa = *reinterpret_cast<const uint4*>(a + i), qb = *reinterpret_cast<const uint4*>(b + i);
-      const __nv_bfloat16* ha = reinterpret_cast<const __nv_bfloat16*>(&qa);
-      const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&qb);
-      __nv_bfloat16 o[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float x = __bfloat162float(ha[k]), y = __bfloat162float(hb[k]);
-        o[k] = __float2bfloat16(i + k < V ? __expf(y - mb) * ib - __expf(x - ma) * ia : 0.f);
-      }
-      *reinterpret_cast<uint4*>(d + i) = *reinterpret_cast<uint4*>(o);
-    }
-  }
-}
-
-
 // out[row, 8g .. 8g+7] = the Philox uniforms the GEMM epilogues draw for (seed, stream, row, g).
 __global__ void philox_uniform_kernel(float* __restrict__ out, long long rows, int groups, int cols,
                                       unsigned long long seed, unsigned int stream, unsigned int row_offset,
@@ -1054,17 +979,6 @@ extern "C" int pd_ci_squash_activity_jobs_bwd(const void* pre, const void* dlowe
       normalize_at_one);
   return PD_CHECK_LAUNCH();
 }
-extern "C" int pd_vocab_kl(const void* lc, const void* lm, void* dlm, float* kl, long long rows, int V,
-                           long long ld, void* stream) {
-  if (ld % 8 != 0 || rows <= 0) return 5;
-  // 512 threads per row: four rows in flight per SM keep the rows being re-read (passes 2 and 3)
-  // within L2 while different rows' load-bound and exp-bound passes still overlap on the SM
-  vocab_kl_kernel<<<static_cast<unsigned>(rows), 512, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(lc), static_cast<const __nv_bfloat16*>(lm),
-      static_cast<__nv_bfloat16*>(dlm), kl, V, ld);
-  return PD_CHECK_LAUNCH();
-}
-
 extern "C" int pd_philox_uniform(float* out, long long rows, int cols, unsigned long long seed, unsigned int stream,
                                  unsigned int row_offset, const unsigned long long* seed_dev, void* stream_v) {
   const int groups = (cols + 7) / 8;

@@ -307,9 +307,9 @@ def vocab_kl_rows(lc: Tensor, lm: Tensor, want_grad: bool, grad_out: Tensor | No
         dlm = torch.empty(rows, lc.stride(0), device=lc.device, dtype=torch.bfloat16)[:, :V]
     lib = _lib()
     lib.pd_vocab_kl.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_longlong,
-                                C.c_void_p]
+                                C.c_void_p, C.c_void_p]
     _check(lib.pd_vocab_kl(lc.data_ptr(), lm.data_ptr(), dlm.data_ptr() if dlm is not None else None, kl.data_ptr(),
-                           rows, V, lc.stride(0), _s()), "vocab_kl")
+                           rows, V, lc.stride(0), nv.status_word().data_ptr(), _s()), "vocab_kl")
     return kl, dlm
 
 

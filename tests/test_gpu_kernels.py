@@ -934,6 +934,32 @@ def test_delta_rule_tiles_against_64_bits(nv, dk, dv, T):
         assert torch.equal(delta_rule.gated_delta_rule(*ins), out)
 
 
+@pytest.mark.parametrize("V", [1003, 8192, 30001, 50277, 151936])
+def test_vocab_kl_rows_over_cluster_sizes(nv, V):
+    """One to eight CTAs per row, rows that do not fill a piece, masked and lowest-value logits. The gradient is a
+    bf16 difference of two probabilities (2^-8 of the larger), the KL a sum of fp32 terms."""
+    from param_decomp_b200.ops.elementwise import vocab_kl_rows
+
+    torch.manual_seed(V)
+    rows, vp = 601, (V + 7) // 8 * 8
+    lc = torch.randn(rows, vp, device="cuda").mul_(3).to(bf)[:, :V]
+    lm = (lc.float() + 0.3 * torch.randn(rows, V, device="cuda")).to(bf)
+    lm = torch.nn.functional.pad(lm, (0, vp - V), value=float("nan"))[:, :V]  # what lies past V is never used
+    low = torch.finfo(bf).min
+    lc[3, : V // 2], lm[3, : V // 2] = low, low
+    lc[4, 1:], lm[4, 1:] = low, low
+    kl, dlm = vocab_kl_rows(lc, lm, want_grad=True)
+    kl2, none = vocab_kl_rows(lc, lm, want_grad=False)
+    a, b = (torch.log_softmax(t.double(), -1) for t in (lc, lm))
+    want = (a.exp() * (a - b)).sum(-1)
+    _done(nv)
+    assert none is None and torch.equal(kl, kl2)
+    assert torch.allclose(kl.double(), want, rtol=1e-4, atol=1e-5)
+    d = b.exp() - a.exp()
+    assert float((dlm.double() - d).abs().max()) <= 2**-8 * float(d.abs().max())
+    assert rel(dlm, d) < 2**-8
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("T,H,Hkv,B", [(128, 2, 1, 1), (256, 3, 3, 2), (640, 12, 4, 30)])
 def test_flash_attention_walks_items(nv, hd, T, H, Hkv, B):
