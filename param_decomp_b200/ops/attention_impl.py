@@ -62,7 +62,7 @@ class FlashAttention(torch.autograd.Function):
         Hkv = k.shape[2]
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         delta = torch.empty(B, H, T, device=q.device, dtype=torch.float32)
-        dq_acc = torch.zeros(B, T, H, hd, device=q.device, dtype=torch.float32)
+        dq_acc = torch.empty(B, T, H, hd, device=q.device, dtype=torch.float32)  # cleared by the first kernel
         rc = _lib().pd_flash_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), d_out.data_ptr(),
                                            lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(),
                                            dk.data_ptr(), dv.data_ptr(), seg.data_ptr() if seg is not None else None,

@@ -22,9 +22,17 @@
 // Backward, one CTA per (128 key rows, kv head, batch), looping over the query heads of the group
 // and the query tiles that see this key tile:
 //     S = Q_i K_j^T, dP = dO_i V_j^T (TMEM) -> P = exp2(S - L), dS = P * (dP - D) * scale (bf16, shared)
-//     dV += P^T dO_i, dK += dS^T Q_i (TMEM, across the whole loop), dQ_i = dS K_j (TMEM -> fp32 atomics)
+//     dV += P^T dO_i, dK += dS^T Q_i (TMEM, across the whole loop), dQ_i = dS K_j (TMEM -> fp32 reductions)
 // P and dS are written once, row-major in the key index, and read both as a K-major operand (dQ) and
 // as an MN-major operand (the transposed products), which the descriptor's major bits allow.
+// Eight elementwise warps, two per TMEM lane quarter, take half of a tile's keys each; four more move dQ out (the
+// reductions of a 128 x 128 dQ keep a warp's load-store path busy for 2000 cycles). The tensor pipe does not wait for a
+// whole tile: S_{i+1} is issued once P_i is stored, dP_{i+1} once dS_i is (hd 64) or once dQ_i, which shares its
+// columns, has been read out (hd 128, 512 TMEM columns). dQ sums in a scratch laid out [b, h, q tile][hd / 4][128 rows][4], so that a warp's 16-byte
+// reductions are one contiguous 512-byte run; a last pass casts it to bf16 rows. The pass over dO and O that forms D
+// also clears that scratch. With one warpgroup that took every step in turn and 16-byte atomics at row pitch, B 64,
+// T 512, 12 heads of 64 took 420 us and B 4, T 2048, 32 / 8 heads of 128 995 us (D, scratch and cast included);
+// now 285 and 570 us. What is left is the chain S -> P -> dP -> dS -> dQ of a tile: 512 columns hold one tile.
 //
 // Every wait is bounded; on a time-out the status word is set and all roles leave.
 //
@@ -48,7 +56,7 @@ struct AttnArgs {
   float* lse;             // [B, H, T] base-2 log-sum-exp of the scaled scores
   // backward only
   const float* delta;     // [B, H, T] rowsum(dO * O)
-  float* dq_accum;        // [B, T, H, hd] fp32, zero on entry
+  float* dq_accum;        // [B, H, T / 128][hd / 4][128][4] fp32
   __nv_bfloat16* dk;      // [B, T, Hkv, hd]
   __nv_bfloat16* dv;
   int* status;
@@ -404,79 +412,106 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
 // ------------------------------------------------------------------------------------------------
 // backward
 // ------------------------------------------------------------------------------------------------
-// D[b, h, t] = sum_d dO * O  (one warp per row)
+// D[b, h, t] = sum_d dO * O, hd / 8 lanes per row; clears the dQ scratch on the way (as many floats as dO has values).
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  float* __restrict__ delta, int B, int T, int H, int hd) {
-  const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);  // (b, t, h)
-  if (row >= static_cast<long long>(B) * T * H) return;
-  const int lane = threadIdx.x & 31;
-  const __nv_bfloat16* po = o + row * hd;
-  const __nv_bfloat16* pd = d_o + row * hd;
+                                  float* __restrict__ delta, float* __restrict__ dq_accum, int B, int T, int H, int hd) {
+  const long long rows = static_cast<long long>(B) * T * H, pieces = rows * (hd / 8);
+  const int lpr = hd / 8;  // 8 or 16: a row never straddles a warp
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;  // 8 values
   float acc = 0.0f;
-  for (int i = lane * 2; i < hd; i += 64) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(po + i));
-    const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(pd + i));
-    acc += a.x * g.x + a.y * g.y;
-  }
+  if (i < pieces) {
+    const uint4 a = *reinterpret_cast<const uint4*>(o + 8 * i), g = *reinterpret_cast<const uint4*>(d_o + 8 * i);
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+    f32x2 t = 0ull;
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) {
-    const long long bt = row / H;
+    for (int k = 0; k < 4; ++k) t = fma2(unpack_bf16_2(aw[k]), unpack_bf16_2(gw[k]), t);
+    const float2 t2 = unpack2(t);
+    acc = t2.x + t2.y;
+    reinterpret_cast<float4*>(dq_accum)[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<float4*>(dq_accum)[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int s = lpr / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if (i < pieces && i % lpr == 0) {
+    const long long row = i / lpr, bt = row / H;
     const int h = static_cast<int>(row % H);
-    const long long b = bt / T, t = bt % T;
-    delta[(b * H + h) * T + t] = acc;
+    delta[(bt / T * H + h) * T + bt % T] = acc;
   }
 }
 
-__global__ void attn_dq_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long n) {
-  for (long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x * 4) {
-    const float4 v = *reinterpret_cast<const float4*>(acc + i);
-    uint2 o;
-    o.x = pack_bf16(v.x, v.y);
-    o.y = pack_bf16(v.z, v.w);
-    *reinterpret_cast<uint2*>(dq + i) = o;
+// [b, h, q tile][hd / 4][128][4] fp32 -> bf16 [B, T, H, hd]: a thread gathers 32 columns of its row; the rows leave
+// through shared memory so that four lanes write a row's 64 bytes together (16 bytes a row and store took 1.6x as long).
+__global__ void __launch_bounds__(kTile) attn_dq_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+                                                             int T, int H, int hd) {
+  __shared__ uint4 rows[kTile][4];
+  const int n_qt = T / kTile, groups = hd / 32;
+  const int cg = static_cast<int>(blockIdx.x % groups);
+  const long long item = blockIdx.x / groups;  // (b, h, qt)
+  const int qt = static_cast<int>(item % n_qt), t = threadIdx.x;
+  const long long bh = item / n_qt;
+  const float4* src = reinterpret_cast<const float4*>(acc) + (item * (hd / 4) + cg * 8) * kTile + t;
+  float4 v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = src[c * kTile];
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    rows[t][c ^ ((t >> 1) & 3)] = make_uint4(pack_bf16(v[2 * c].x, v[2 * c].y), pack_bf16(v[2 * c].z, v[2 * c].w),
+                                             pack_bf16(v[2 * c + 1].x, v[2 * c + 1].y), pack_bf16(v[2 * c + 1].z, v[2 * c + 1].w));
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = k * 32 + (t >> 2), c = t & 3;
+    __nv_bfloat16* dst = dq + ((bh / H * T + qt * kTile + r) * H + bh % H) * hd + cg * 32 + 8 * c;
+    *reinterpret_cast<uint4*>(dst) = rows[r][c ^ ((r >> 1) & 3)];
   }
 }
+
+constexpr int kBwdEwThreads = 256;                     // two elementwise warps per TMEM lane quarter
+constexpr int kBwdDqThreads = 128;                     // four warps that move dQ out
+constexpr int kBwdThreads = kBwdEwThreads + kBwdDqThreads + 64;  // then the producer and the MMA issuer
 
 template <int HD>
 struct BwdPlan {
   static constexpr int kTileBytes = kTile * HD * 2;  // K, V, Q or dO tile
-  static constexpr int kStages = HD == 64 ? 2 : 1;   // Q / dO ring
+  static constexpr int kDoStages = HD == 64 ? 2 : 1;
   static constexpr int kPBytes = kTile * kTile * 2;
-  static constexpr int kTotal = 2 * kTileBytes + 2 * kStages * kTileBytes + 2 * kPBytes + 1024 + 1024;
-  // TMEM: [0,128) S, later dQ; [128,256) dP; [256,256+HD) dV; [256+HD, 256+2HD) dK
+  static constexpr int kTotal = (2 + 2 /*Q ring*/ + kDoStages) * kTileBytes + 2 * kPBytes + 1024 /*align*/ + 1024 /*barriers, ids*/;
   static constexpr uint32_t kTmemCols = 512;
+  // S [0, 128), dP [128, 256), dV, dK, then dQ in columns of its own (hd 64) or over dP (hd 128)
+  static constexpr bool kOwnDq = HD == 64;
+  static constexpr uint32_t kDv = 256, kDk = 256 + HD, kDq = kOwnDq ? 384 : 128;
 };
 
 template <int HD>
-__global__ void __launch_bounds__(kFwdThreads, 1) attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ,
+__global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                    const __grid_constant__ CUtensorMap tmK,
                                                                    const __grid_constant__ CUtensorMap tmV,
                                                                    const __grid_constant__ CUtensorMap tmdO,
                                                                    const AttnArgs args) {
   using Plan = BwdPlan<HD>;
-  constexpr int kStages = Plan::kStages;
+  constexpr int kDoStages = Plan::kDoStages;
   constexpr int kKB = HD / 64;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sm_k = base;
   const uint32_t sm_v = sm_k + Plan::kTileBytes;
   const uint32_t sm_q = sm_v + Plan::kTileBytes;
-  const uint32_t sm_do = sm_q + kStages * Plan::kTileBytes;
-  const uint32_t sm_p = sm_do + kStages * Plan::kTileBytes;
+  const uint32_t sm_do = sm_q + 2 * Plan::kTileBytes;
+  const uint32_t sm_p = sm_do + kDoStages * Plan::kTileBytes;
   const uint32_t sm_ds = sm_p + Plan::kPBytes;
   const uint32_t sm_bar = sm_ds + Plan::kPBytes;
-  // barriers: kv_full, qdo_full[2], qdo_empty[2], sdp_full, pds_full, dq_full, dq_empty, final
   const uint32_t bar_kv = sm_bar;
-  const uint32_t bar_qf = bar_kv + 8, bar_qe = bar_qf + 16;
-  const uint32_t bar_sdp = bar_qe + 16, bar_pds = bar_sdp + 8, bar_dqf = bar_pds + 8, bar_dqe = bar_dqf + 8;
+  const uint32_t bar_qf = bar_kv + 8, bar_qe = bar_qf + 16;    // Q ring full / empty [2]
+  const uint32_t bar_gf = bar_qe + 16, bar_ge = bar_gf + 16;   // dO ring full / empty [2]
+  const uint32_t bar_s = bar_ge + 16, bar_dp = bar_s + 8;      // S, dP formed
+  const uint32_t bar_pf = bar_dp + 8, bar_pe = bar_pf + 8;     // P stored (S read) / consumed
+  const uint32_t bar_df = bar_pe + 8, bar_de = bar_df + 8;     // dS stored (dP read) / consumed
+  const uint32_t bar_dqf = bar_de + 8, bar_dqe = bar_dqf + 8;  // dQ formed / read out
   const uint32_t bar_fin = bar_dqe + 8;
   const uint32_t tmem_slot = bar_fin + 8;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + (tmem_slot + 4 - base));
-  int* seg_k = reinterpret_cast<int*>(gbase + (sm_bar + 256 - base));
+  int* seg_k = reinterpret_cast<int*>(gbase + (sm_bar + 256 - base));  // [128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qt = args.T / kTile;
@@ -491,11 +526,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_bwd_kernel(const __grid_c
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_qf + 8 * s, 1);
       mbar_init(bar_qe + 8 * s, 1);
+      mbar_init(bar_gf + 8 * s, 1);
+      mbar_init(bar_ge + 8 * s, 1);
     }
-    mbar_init(bar_sdp, 1);
-    mbar_init(bar_pds, kSoftmaxThreads);
+    mbar_init(bar_s, 1);
+    mbar_init(bar_dp, 1);
+    mbar_init(bar_pf, kBwdEwThreads);
+    mbar_init(bar_pe, 1);
+    mbar_init(bar_df, kBwdEwThreads);
+    mbar_init(bar_de, 1);
     mbar_init(bar_dqf, 1);
-    mbar_init(bar_dqe, kSoftmaxThreads);
+    mbar_init(bar_dqe, kBwdDqThreads);
     mbar_init(bar_fin, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -504,7 +545,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_bwd_kernel(const __grid_c
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmdO);
   }
-  if (warp == 5) {
+  if (threadIdx.x < kTile && args.segment_ids)
+    seg_k[threadIdx.x] = args.segment_ids[static_cast<long long>(b) * args.T + kt * kTile + threadIdx.x];
+  if (warp == 13) {
     tmem_alloc(tmem_slot, Plan::kTmemCols);
     tmem_relinquish();
   }
@@ -513,10 +556,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_bwd_kernel(const __grid_c
   tc_fence_after();
   const uint32_t tmem_s = *tmem_slot_ptr;
   const uint32_t tmem_dp = tmem_s + 128;
-  const uint32_t tmem_dv = tmem_s + 256;
-  const uint32_t tmem_dk = tmem_dv + HD;
+  const uint32_t tmem_dv = tmem_s + Plan::kDv, tmem_dk = tmem_s + Plan::kDk, tmem_dq = tmem_s + Plan::kDq;
 
-  if (warp == 4) {
+  if (warp == 12) {
+    // ---------------- TMA producer ----------------
     if (elect_one_sync()) {
       mbar_expect_tx(bar_kv, 2 * Plan::kTileBytes);
       for (int c = 0; c < kKB; ++c) {
@@ -525,185 +568,252 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_bwd_kernel(const __grid_c
       }
     }
     for (int it = 0; it < n_it; ++it) {
-      const int st = it % kStages;
-      const uint32_t ph = static_cast<uint32_t>((it / kStages) & 1);
-      if (!mbar_wait_warp(bar_qe + 8 * st, ph ^ 1, abort_flag)) {
+      const int h = hk * group + it / per_head, qt = qt_lo + it % per_head;
+      auto load = [&](uint32_t full, uint32_t empty, uint32_t dst, const CUtensorMap* tm, int stages) {
+        const int st = it % stages;
+        if (!mbar_wait_warp(empty + 8 * st, static_cast<uint32_t>((it / stages) & 1) ^ 1, abort_flag)) return false;
+        if (elect_one_sync()) {
+          mbar_expect_tx(full + 8 * st, Plan::kTileBytes);
+          for (int c = 0; c < kKB; ++c)
+            tma_load_3d(dst + st * Plan::kTileBytes + c * (kTile * 128), tm, full + 8 * st, h * HD + 64 * c, qt * kTile, b);
+        }
+        return true;
+      };
+      if (!load(bar_qf, bar_qe, sm_q, &tmQ, 2) || !load(bar_gf, bar_ge, sm_do, &tmdO, kDoStages)) {
         if (lane == 0) atomicCAS(args.status, 0, kTimeoutProducer);
         break;
       }
-      const int h = hk * group + it / per_head;
-      const int qt = qt_lo + it % per_head;
-      if (elect_one_sync()) {
-        mbar_expect_tx(bar_qf + 8 * st, 2 * Plan::kTileBytes);
-        for (int c = 0; c < kKB; ++c) {
-          tma_load_3d(sm_q + st * Plan::kTileBytes + c * (kTile * 128), &tmQ, bar_qf + 8 * st, h * HD + 64 * c,
-                      qt * kTile, b);
-          tma_load_3d(sm_do + st * Plan::kTileBytes + c * (kTile * 128), &tmdO, bar_qf + 8 * st, h * HD + 64 * c,
-                      qt * kTile, b);
-        }
-      }
     }
-  } else if (warp == 5) {
-    {
-      constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);   // Q K^T, dO V^T
-      constexpr uint32_t idesc_t = make_idesc_bf16(kTile, HD, 1, 1);      // P^T dO, dS^T Q
-      constexpr uint32_t idesc_q = make_idesc_bf16(kTile, HD, 0, 1);      // dS K
-      bool ok = mbar_wait_warp(bar_kv, 0, abort_flag);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int st = it % kStages;
-        if (!mbar_wait_warp(bar_qf + 8 * st, static_cast<uint32_t>((it / kStages) & 1), abort_flag)) { ok = false; break; }
-        // the softmax warps have read dQ of the previous iteration out of the S columns
-        if (!mbar_wait_warp(bar_dqe, static_cast<uint32_t>((it & 1) ^ 1), abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t q_s = sm_q + st * Plan::kTileBytes, do_s = sm_do + st * Plan::kTileBytes;
-        if (elect_one_sync()) {
+  } else if (warp == 13) {
+    // ---------------- MMA issuer ----------------
+    constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);   // Q K^T, dO V^T
+    constexpr uint32_t idesc_t = make_idesc_bf16(kTile, HD, 1, 1);      // P^T dO, dS^T Q
+    constexpr uint32_t idesc_q = make_idesc_bf16(kTile, HD, 0, 1);      // dS K
+    auto wait = [&](uint32_t bar, int count) { return mbar_wait_warp(bar, static_cast<uint32_t>(count & 1), abort_flag); };
+    // D = A B^T of two K-major tiles (S and dP)
+    auto issue_nt = [&](uint32_t d, uint32_t a_s, uint32_t b_s, uint32_t done) {
+      if (elect_one_sync()) {
 #pragma unroll
-          for (int c = 0; c < kKB; ++c) {
-            const uint64_t qd = make_smem_desc(q_s + c * (kTile * 128), 16, 1024);
-            const uint64_t kd = make_smem_desc(sm_k + c * (kTile * 128), 16, 1024);
-            const uint64_t dod = make_smem_desc(do_s + c * (kTile * 128), 16, 1024);
-            const uint64_t vd = make_smem_desc(sm_v + c * (kTile * 128), 16, 1024);
+        for (int c = 0; c < kKB; ++c) {
+          const uint64_t ad = make_smem_desc(a_s + c * (kTile * 128), 16, 1024);
+          const uint64_t bd = make_smem_desc(b_s + c * (kTile * 128), 16, 1024);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              umma_bf16(tmem_s, qd + k * 2, kd + k * 2, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
-              umma_bf16(tmem_dp, dod + k * 2, vd + k * 2, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
-            }
-          }
-          umma_commit(bar_sdp);
+          for (int k = 0; k < 4; ++k) umma_bf16(d, ad + k * 2, bd + k * 2, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
         }
-        if (!mbar_wait_warp(bar_pds, static_cast<uint32_t>(it & 1), abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one_sync()) {
-          // transposed products: A = P or dS read MN-major (K = query rows), B = dO or Q read MN-major
-          const uint64_t pt = make_smem_desc(sm_p, kTile * 128, 1024);
-          const uint64_t dst = make_smem_desc(sm_ds, kTile * 128, 1024);
-          const uint64_t dob = make_smem_desc(do_s, kTile * 128, 1024);
-          const uint64_t qb = make_smem_desc(q_s, kTile * 128, 1024);
-#pragma unroll
-          for (int k = 0; k < kTile / 16; ++k) {
-            umma_bf16(tmem_dv, pt + k * (2048 >> 4), dob + k * (2048 >> 4), idesc_t, (it > 0 || k > 0) ? 1u : 0u);
-            umma_bf16(tmem_dk, dst + k * (2048 >> 4), qb + k * (2048 >> 4), idesc_t, (it > 0 || k > 0) ? 1u : 0u);
-          }
-          // dQ_i = dS K_j: A = dS K-major in the key index, B = K_j read MN-major (K = key rows)
-          const uint64_t kb_ = make_smem_desc(sm_k, kTile * 128, 1024);
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const uint64_t dsd = make_smem_desc(sm_ds + c * (kTile * 128), 16, 1024);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16(tmem_s, dsd + k * 2, kb_ + (c * 4 + k) * (2048 >> 4), idesc_q, (c > 0 || k > 0) ? 1u : 0u);
-          }
-          umma_commit(bar_qe + 8 * st);
-          umma_commit(bar_dqf);
-        }
+        umma_commit(done);
       }
-      if (ok && elect_one_sync()) umma_commit(bar_fin);
-      if (!ok && lane == 0) atomicCAS(args.status, 0, kTimeoutMma);
+    };
+    // D (+)= A^T B: A = P or dS read MN-major (K = query rows), B = dO or Q read MN-major
+    auto issue_tn = [&](uint32_t d, uint32_t a_s, uint32_t b_s, bool first) {
+      const uint64_t ad = make_smem_desc(a_s, kTile * 128, 1024), bd = make_smem_desc(b_s, kTile * 128, 1024);
+#pragma unroll
+      for (int k = 0; k < kTile / 16; ++k)
+        umma_bf16(d, ad + k * (2048 >> 4), bd + k * (2048 >> 4), idesc_t, (!first || k > 0) ? 1u : 0u);
+    };
+    auto issue_s = [&](int it) {
+      if (!mbar_wait_warp(bar_qf + 8 * (it & 1), static_cast<uint32_t>((it >> 1) & 1), abort_flag)) return false;
+      tc_fence_after();
+      issue_nt(tmem_s, sm_q + (it & 1) * Plan::kTileBytes, sm_k, bar_s);
+      return true;
+    };
+    auto issue_dp = [&](int it) {
+      const int st = it % kDoStages;
+      if (!mbar_wait_warp(bar_gf + 8 * st, static_cast<uint32_t>((it / kDoStages) & 1), abort_flag)) return false;
+      tc_fence_after();
+      issue_nt(tmem_dp, sm_do + st * Plan::kTileBytes, sm_v, bar_dp);
+      return true;
+    };
+    bool ok = mbar_wait_warp(bar_kv, 0, abort_flag);
+    if (n_it > 0) ok = ok && issue_s(0) && issue_dp(0);
+    for (int it = 0; it < n_it && ok; ++it) {
+      const uint32_t q_s = sm_q + (it & 1) * Plan::kTileBytes;
+      const int g_st = it % kDoStages;
+      ok = wait(bar_pf, it);
+      if (!ok) break;
+      tc_fence_after();
+      if (it + 1 < n_it && !issue_s(it + 1)) { ok = false; break; }
+      if (elect_one_sync()) {
+        issue_tn(tmem_dv, sm_p, sm_do + g_st * Plan::kTileBytes, it == 0);
+        umma_commit(bar_pe);
+        umma_commit(bar_ge + 8 * g_st);
+      }
+      ok = wait(bar_df, it);
+      if (!ok) break;
+      tc_fence_after();
+      if (Plan::kOwnDq) {
+        if (it + 1 < n_it && !issue_dp(it + 1)) { ok = false; break; }
+        if (it > 0 && !wait(bar_dqe, it - 1)) { ok = false; break; }
+        tc_fence_after();
+      }
+      if (elect_one_sync()) {
+        // dQ_i = dS K_j: A = dS K-major in the key index, B = K_j read MN-major (K = key rows)
+        const uint64_t kb_ = make_smem_desc(sm_k, kTile * 128, 1024);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const uint64_t dsd = make_smem_desc(sm_ds + c * (kTile * 128), 16, 1024);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_bf16(tmem_dq, dsd + k * 2, kb_ + (c * 4 + k) * (2048 >> 4), idesc_q, (c > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(bar_dqf);
+        issue_tn(tmem_dk, sm_ds, q_s, it == 0);
+        umma_commit(bar_de);
+        umma_commit(bar_qe + 8 * (it & 1));
+      }
+      if (!Plan::kOwnDq && it + 1 < n_it && (!wait(bar_dqe, it) || !issue_dp(it + 1))) { ok = false; break; }
+    }
+    if (ok && elect_one_sync()) umma_commit(bar_fin);
+    if (!ok && lane == 0) atomicCAS(args.status, 0, kTimeoutMma);
+  } else if (warp >= 8) {
+    // ---------------- dQ -> fp32 scratch (other key tiles add to the same rows) ----------------
+    const int row = threadIdx.x - kBwdEwThreads;
+    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    int item = (b * args.H + hk * group) * n_qt + qt_lo, qi = 0;  // (b, h, q tile), and the tile's count in this head
+    for (int it = 0; it < n_it; ++it) {
+      float4* dst = reinterpret_cast<float4*>(args.dq_accum) + static_cast<long long>(item) * (HD / 4) * kTile + row;
+      if (++qi == per_head) {  // next head of the group
+        qi = 0;
+        item += qt_lo;
+      }
+      ++item;
+      if (!mbar_wait_warp(bar_dqf, static_cast<uint32_t>(it & 1), abort_flag)) {
+        if (lane == 0) atomicCAS(args.status, 0, kTimeoutEpilogue);
+        break;
+      }
+      tc_fence_after();
+      uint32_t r[HD / 32][32];
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c) tmem_ld_32x32(tmem_dq + lane_base + c * 32, r[c]);
+      tmem_ld_wait();
+      tc_fence_before();
+      mbar_arrive(bar_dqe);
+#pragma unroll
+      for (int c = 0; c < HD / 32; ++c)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + (c * 8 + i) * kTile),
+                       "f"(__uint_as_float(r[c][4 * i])), "f"(__uint_as_float(r[c][4 * i + 1])),
+                       "f"(__uint_as_float(r[c][4 * i + 2])), "f"(__uint_as_float(r[c][4 * i + 3]))
+                       : "memory");
     }
   } else {
-    const int row = threadIdx.x;
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    if (args.segment_ids) seg_k[row] = args.segment_ids[b * args.T + kt * kTile + row];
-    named_barrier_softmax();
+    // ---------------- elementwise: query row = TMEM lane, `half` picks 64 keys of the tile ----------------
+    const int row = threadIdx.x & (kTile - 1), half = warp >> 2;
+    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = true;
-    uint32_t r[32], g[32];
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int h = hk * group + it / per_head;
-      const int qt = qt_lo + it % per_head;
-      const int q_idx = qt * kTile + row;
-      const long long stat = (static_cast<long long>(b) * args.H + h) * args.T + q_idx;
-      const float L = args.lse[stat];
-      const float Dq = args.delta[stat];
-      const int seg_q = args.segment_ids ? args.segment_ids[b * args.T + q_idx] : 0;
-      const bool diag = args.causal && qt == kt;
-      if (!mbar_wait(bar_sdp, static_cast<uint32_t>(it & 1), abort_flag)) { ok = false; break; }
+    auto wait = [&](uint32_t bar, int count) {
+      ok = mbar_wait_warp(bar, static_cast<uint32_t>(count & 1), abort_flag);
+      return ok;
+    };
+    const f32x2 scale_log2 = pk2(args.scale_log2, args.scale_log2), scale = pk2(args.scale, args.scale);
+    const uint32_t blk_p = sm_p + half * (kTile * 128), blk_ds = sm_ds + half * (kTile * 128);
+    float next_L = 0.0f, next_D = 0.0f;
+    int next_seg = 0;
+    const long long stat_h = (static_cast<long long>(b) * args.H + hk * group) * args.T + row;
+    const int* seg_q_row = args.segment_ids ? args.segment_ids + static_cast<long long>(b) * args.T + row : nullptr;
+    auto load_stats = [&](int head, int tile) {  // an iteration ahead: their latency stays off the chain
+      const long long stat = stat_h + static_cast<long long>(head) * args.T + tile * kTile;
+      next_L = args.lse[stat];
+      next_D = args.delta[stat];
+      if (seg_q_row) next_seg = seg_q_row[tile * kTile];
+    };
+    int head_n = 0, qt_n = qt_lo;  // of the next iteration
+    load_stats(0, qt_n);
+    for (int it = 0; it < n_it; ++it) {
+      const int qt = qt_n, seg_q = next_seg;
+      const f32x2 negL = pk2(-next_L, -next_L), negD = pk2(-next_D, -next_D);
+      if (++qt_n == n_qt) {
+        qt_n = qt_lo;
+        ++head_n;
+      }
+      if (it + 1 < n_it) load_stats(head_n, qt_n);
+      if (!wait(bar_s, it)) break;
       tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        tmem_ld_32x32(tmem_s + lane_base + c * 32, r);
-        tmem_ld_32x32(tmem_dp + lane_base + c * 32, g);
-        tmem_ld_wait();
-        uint32_t pp[16], dd[16];
+      uint32_t r[2][32];  // scores, then probabilities
+#pragma unroll
+      for (int c = 0; c < 2; ++c) tmem_ld_32x32(tmem_s + lane_base + half * 64 + c * 32, r[c]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p2[2], d2[2];
+          const float2 x = unpack2(fma2(pk2u(r[c][i], r[c][i + 1]), scale_log2, negL));
+          r[c][i] = __float_as_uint(fast_exp2(x.x));
+          r[c][i + 1] = __float_as_uint(fast_exp2(x.y));
+        }
+      if (args.causal && qt == kt) {
+        const int lim = row - half * 64;  // last key column of this half that the row sees
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int col = c * 32 + i + e;  // key index inside the tile
-            const bool keep = (!diag || col <= row) && (!args.segment_ids || seg_k[col] == seg_q);
-            const float p = keep ? fast_exp2(__uint_as_float(r[i + e]) * args.scale_log2 - L) : 0.0f;
-            p2[e] = p;
-            d2[e] = p * (__uint_as_float(g[i + e]) - Dq) * args.scale;
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i > lim) r[c][i] = 0u;
+      }
+      if (args.segment_ids) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const int4 id = *reinterpret_cast<const int4*>(seg_k + half * 64 + c * 32 + i);
+            if (id.x != seg_q) r[c][i] = 0u;
+            if (id.y != seg_q) r[c][i + 1] = 0u;
+            if (id.z != seg_q) r[c][i + 2] = 0u;
+            if (id.w != seg_q) r[c][i + 3] = 0u;
           }
-          pp[i >> 1] = pack_bf16(p2[0], p2[1]);
-          dd[i >> 1] = pack_bf16(d2[0], d2[1]);
-        }
-        const uint32_t off = (c >> 1) * (kTile * 128);
+      }
+      if (it > 0 && !wait(bar_pe, it - 1)) break;
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const uint32_t a = swz(row, (c & 1) * 4 + q4);
-          st_shared_v4(sm_p + off + a, make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]));
-          st_shared_v4(sm_ds + off + a, make_uint4(dd[4 * q4], dd[4 * q4 + 1], dd[4 * q4 + 2], dd[4 * q4 + 3]));
-        }
+      for (int g = 0; g < 8; ++g) {
+        const uint32_t* v = &r[g >> 2][(g & 3) * 8];
+        st_shared_v4(blk_p + swz(row, g), make_uint4(pack_bf16_2(pk2u(v[0], v[1])), pack_bf16_2(pk2u(v[2], v[3])),
+                                                     pack_bf16_2(pk2u(v[4], v[5])), pack_bf16_2(pk2u(v[6], v[7]))));
       }
       tc_fence_before();
       fence_proxy_async_smem();
-      mbar_arrive(bar_pds);
-      // dQ_i tile -> fp32 accumulation buffer (other key tiles add to the same rows)
-      if (!mbar_wait(bar_dqf, static_cast<uint32_t>(it & 1), abort_flag)) { ok = false; break; }
+      mbar_arrive(bar_pf);
+      if (!wait(bar_dp, it)) break;
       tc_fence_after();
-      float* dq_row = args.dq_accum + ((static_cast<long long>(b) * args.T + q_idx) * args.H + h) * HD;
-#pragma unroll 1
-      for (int c = 0; c < HD / 32; ++c) {
-        tmem_ld_32x32(tmem_s + lane_base + c * 32, r);
-        tmem_ld_wait();
+      if (it > 0 && !wait(bar_de, it - 1)) break;
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          atomicAdd(reinterpret_cast<float4*>(dq_row + c * 32 + i),
-                    make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]),
-                                __uint_as_float(r[i + 3])));
+      for (int c = 0; c < 2; ++c) {
+        uint32_t g[32];
+        tmem_ld_32x32(tmem_dp + lane_base + half * 64 + c * 32, g);
+        tmem_ld_wait();
+        uint32_t d[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          d[i] = pack_bf16_2(mul2(mul2(pk2u(r[c][2 * i], r[c][2 * i + 1]), add2(pk2u(g[2 * i], g[2 * i + 1]), negD)), scale));
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4)
+          st_shared_v4(blk_ds + swz(row, c * 4 + q4), make_uint4(d[4 * q4], d[4 * q4 + 1], d[4 * q4 + 2], d[4 * q4 + 3]));
       }
       tc_fence_before();
-      mbar_arrive(bar_dqe);
+      fence_proxy_async_smem();
+      mbar_arrive(bar_df);
     }
-    if (ok) {
-      if (n_it > 0) {
-        if (!mbar_wait(bar_fin, 0, abort_flag)) ok = false;
-      }
-      if (ok) {
-        tc_fence_after();
-        const long long krow = ((static_cast<long long>(b) * args.T + kt * kTile + row) * args.Hkv + hk) * HD;
+    if (ok && n_it > 0) wait(bar_fin, 0);
+    if (ok) {  // dV by the first four warps, dK by the others
+      tc_fence_after();
+      const long long krow = ((static_cast<long long>(b) * args.T + kt * kTile + row) * args.Hkv + hk) * HD;
+      __nv_bfloat16* dst = (half == 0 ? args.dv : args.dk) + krow;
+      const uint32_t src = (half == 0 ? tmem_dv : tmem_dk) + lane_base;
 #pragma unroll 1
-        for (int which = 0; which < 2; ++which) {
-          __nv_bfloat16* dst = (which == 0 ? args.dv : args.dk) + krow;
-          const uint32_t src = (which == 0 ? tmem_dv : tmem_dk) + lane_base;
-#pragma unroll 1
-          for (int c = 0; c < HD / 32; ++c) {
-            if (n_it > 0) {
-              tmem_ld_32x32(src + c * 32, r);
-              tmem_ld_wait();
-            } else {
+      for (int c = 0; c < HD / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32(src + c * 32, r);
+        tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0u;
-            }
-#pragma unroll
-            for (int q8 = 0; q8 < 4; ++q8) {
-              uint4 v;
-              v.x = pack_bf16(__uint_as_float(r[8 * q8]), __uint_as_float(r[8 * q8 + 1]));
-              v.y = pack_bf16(__uint_as_float(r[8 * q8 + 2]), __uint_as_float(r[8 * q8 + 3]));
-              v.z = pack_bf16(__uint_as_float(r[8 * q8 + 4]), __uint_as_float(r[8 * q8 + 5]));
-              v.w = pack_bf16(__uint_as_float(r[8 * q8 + 6]), __uint_as_float(r[8 * q8 + 7]));
-              *reinterpret_cast<uint4*>(dst + c * 32 + 8 * q8) = v;
-            }
-          }
-        }
+        for (int g = 0; g < 4; ++g)
+          *reinterpret_cast<uint4*>(dst + c * 32 + 8 * g) =
+              make_uint4(pack_bf16_2(pk2u(r[8 * g], r[8 * g + 1])), pack_bf16_2(pk2u(r[8 * g + 2], r[8 * g + 3])),
+                         pack_bf16_2(pk2u(r[8 * g + 4], r[8 * g + 5])), pack_bf16_2(pk2u(r[8 * g + 6], r[8 * g + 7])));
       }
     }
     if (!ok) atomicCAS(args.status, 0, kTimeoutEpilogue);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) tmem_dealloc(tmem_s, Plan::kTmemCols);
+  if (warp == 13) tmem_dealloc(tmem_s, Plan::kTmemCols);
 }
 
 template <int HD>
@@ -732,7 +842,7 @@ int launch_bwd(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
     configured = true;
   }
   dim3 grid(a.T / kTile, a.Hkv, a.B);
-  kern<<<grid, kFwdThreads, BwdPlan<HD>::kTotal, st>>>(q, k, v, d_o, a);
+  kern<<<grid, kBwdThreads, BwdPlan<HD>::kTotal, st>>>(q, k, v, d_o, a);
   return cudaGetLastError() == cudaSuccess ? 0 : 400;
 }
 
@@ -759,8 +869,8 @@ extern "C" int pd_flash_attention_fwd(const void* q, const void* k, const void* 
   return hd == 64 ? launch_fwd<64>(tq, tk, tv, a, st) : launch_fwd<128>(tq, tk, tv, a, st);
 }
 
-// `delta` [B, H, T] fp32 and `dq_accum` [B, T, H, hd] fp32 are scratch supplied by the caller;
-// `dq_accum` must be zero on entry.
+// `delta` [B, H, T] fp32 and `dq_accum` (B T H hd floats) are scratch supplied by the caller, contents irrelevant;
+// out, d_out and dq_accum on 16-byte boundaries.
 extern "C" int pd_flash_attention_bwd(const void* q, const void* k, const void* v, const void* out, const void* d_out,
                                       const float* lse, float* delta, float* dq_accum, void* dq, void* dk, void* dv,
                                       const int* segment_ids, int B, int T, int H, int Hkv, int hd, int causal,
@@ -773,9 +883,10 @@ extern "C" int pd_flash_attention_bwd(const void* q, const void* k, const void* 
   if ((rc = encode_bthd(&tv, v, B, T, Hkv, hd)) != 0) return 1000 + rc;
   if ((rc = encode_bthd(&tdo, d_out, B, T, H, hd)) != 0) return 1000 + rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long rows = static_cast<long long>(B) * T * H;
-  attn_delta_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, B, T, H, hd);
+  const long long rows = static_cast<long long>(B) * T * H, pieces = rows * (hd / 8);
+  if ((pieces + 255) / 256 > 0x7FFFFFFF || rows / kTile > 0x3FFFFFFF) return kBadArgument;
+  attn_delta_kernel<<<static_cast<unsigned>((pieces + 255) / 256), 256, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), delta, dq_accum, B, T, H, hd);
   AttnArgs a{};
   a.B = B; a.T = T; a.H = H; a.Hkv = Hkv; a.causal = causal;
   a.scale = 1.0f / sqrtf(static_cast<float>(hd));
@@ -789,8 +900,7 @@ extern "C" int pd_flash_attention_bwd(const void* q, const void* k, const void* 
   a.status = status;
   rc = hd == 64 ? launch_bwd<64>(tq, tk, tv, tdo, a, st) : launch_bwd<128>(tq, tk, tv, tdo, a, st);
   if (rc != 0) return rc;
-  const long long n = rows * hd;
-  attn_dq_cast_kernel<<<static_cast<unsigned>(std::min<long long>((n / 4 + 255) / 256, 148 * 16)), 256, 0, st>>>(
-      dq_accum, static_cast<__nv_bfloat16*>(dq), n);
+  attn_dq_cast_kernel<<<static_cast<unsigned>(rows / kTile * (hd / 32)), kTile, 0, st>>>(
+      dq_accum, static_cast<__nv_bfloat16*>(dq), T, H, hd);
   return cudaGetLastError() == cudaSuccess ? 0 : 400;
 }
