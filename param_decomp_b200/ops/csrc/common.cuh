@@ -448,7 +448,7 @@ inline int encode_tmap(CUtensorMap* tm, const void* base, int elem_size, bool is
   if (fn == nullptr) return 100;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return 101;
   if ((ld * elem_size) % 16 != 0) return 102;
-  if (box_inner * elem_size != 128) return 103;
+  if (box_inner * elem_size != 128 && box_inner * elem_size != 64) return 103;  // 128- or 64-byte swizzle rows
   if (box_rows > 256) return 104;
   CUtensorMapDataType dt = elem_size == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                           : (is_float ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
@@ -462,15 +462,16 @@ inline int encode_tmap(CUtensorMap* tm, const void* base, int elem_size, bool is
   cuuint32_t box[3] = {box_inner, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   const cuuint32_t rank = 3;
+  const CUtensorMapSwizzle swizzle = box_inner * elem_size == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
   CUresult r = fn(tm, dt, rank, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r == CUDA_ERROR_INVALID_CONTEXT) {
     // The driver call needs a context current on THIS host thread (e.g. a fresh autograd worker);
     // a no-op runtime call binds the device's primary context, then the encode is retried once.
     cudaFree(nullptr);
     r = fn(tm, dt, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   }
   return r == CUDA_SUCCESS ? 0 : 200 + static_cast<int>(r);
 }

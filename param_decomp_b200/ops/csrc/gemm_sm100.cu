@@ -11,7 +11,7 @@
 // Two K-phases let one accumulator take  (xV .* coef) U  +  (d .* x) W^T  without a second pass:
 // phase 0 walks the component axis, phase 1 walks d_in, and the sum never leaves TMEM.
 //
-// Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + single-thread MMA issuer,
+// Warp roles (320 threads; 576 in the TMA-fed mask form, warps 2..17 = epilogue): warp 0 = TMA producer, warp 1 = TMEM owner + single-thread MMA issuer,
 // warps 2..9 = epilogue. A warp may only read the TMEM lane quarter warp_id % 4, so two warps share
 // each quarter and take alternate output boxes; with short K (d_in = 768) the epilogue is the
 // longer half of a tile and needs the issue slots of all four schedulers. Two accumulators of BN
@@ -33,8 +33,8 @@
 // The mask epilogues come in two forms. NOUT = 1 / 2: each epilogue thread reads its row's ci / H values with
 // plain global loads (row-strided: 32 cache lines per warp request) and writes its mask gradient the same way;
 // this form serves row-mapped (routed) products. NOUT = 4, the TMA-fed form for dense sites: ci and H arrive as
-// 32-row x 64-column boxes by TMA into a two-slot ring of shared-memory boxes per epilogue warp (issued one
-// unit ahead), every thread reads its own 128-byte row of the swizzled box, writes its results IN PLACE
+// 32-row x 32-column boxes by TMA into a two-slot ring of shared-memory boxes per epilogue warp (issued one
+// unit ahead), every thread reads its own 64-byte row of the swizzled box, writes its results IN PLACE
 // (ci box -> A or dH, H box -> mask gradient or the H output) and the boxes leave by TMA store. No global
 // load or store instruction is left in the epilogue: L1 wavefronts drop from 32 to 4 per 16-byte request.
 //
@@ -45,8 +45,15 @@ namespace pd {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int kNumEpiWarps = 8;
-constexpr int kNumThreads = 32 * (2 + kNumEpiWarps);
+// Epilogue warps: two per TMEM lane quarter; four in the TMA-fed mask form, whose arithmetic (about 16 instructions an
+// element, chains of seven Philox rounds) two warps per scheduler issue at a quarter of the rate. 32768 x 768 -> 4096
+// components: mask gradient 306 -> 281 us; the forward stays at 262 us, with or without the Philox draw (259): its
+// operand loads and box traffic share L2 with 0.8 GB of results, 1085 cycles a K block against 512 for the MMAs. One slot
+// per warp and five pipeline stages instead of two and three: 281 / 307 us.
+template <int NOUT>
+constexpr int kEpiWarps = NOUT == 4 ? 16 : 8;
+template <int NOUT>
+constexpr int kThreads = 32 * (2 + kEpiWarps<NOUT>);
 constexpr int kGatherChunk = 16384;  // bytes per bulk copy of the all-gather CTAs
 constexpr int kGatherSlotsMax = 12;
 constexpr int kMaxPeers = 8;
@@ -57,6 +64,7 @@ struct PeerMaps {
 constexpr int kGroupM = 16;
 constexpr int kStageBytesA = BM * BK * 2;  // 16 KiB
 constexpr int kOutBoxBytes = 32 * 128;     // one 32-row x 128-byte staging box
+constexpr int kFedBoxBytes = 32 * 64;      // one 32-row x 32-column bf16 box of the TMA-fed mask epilogue
 
 enum Epi : int { EPI_PLAIN = 0, EPI_MASK_FWD = 1, EPI_MASK_BWD = 2, EPI_FAITH = 3 };
 enum Act : int { ACT_NONE = 0, ACT_GELU = 1, ACT_SILU = 2, ACT_RELU = 3 };
@@ -129,11 +137,11 @@ template <int BN, int NOUT, int CG = 1>
 struct SmemPlan {
   static constexpr int kStageBytesB = BN * BK * 2 / CG;  // a CTA pair splits the B tile
   static constexpr int kStageBytes = kStageBytesA + kStageBytesB;
-  static constexpr int kOutBytes = kNumEpiWarps * NOUT * kOutBoxBytes;
+  static constexpr int kOutBytes = NOUT == 4 ? kEpiWarps<NOUT> * 4 * kFedBoxBytes : kEpiWarps<NOUT> * NOUT * kOutBoxBytes;
   static constexpr int kBarrierBytes = 512;  // pipeline + accumulator barriers, then two operand barriers per epilogue warp
   static constexpr int kBudget = 227 * 1024 - 1024 /*alignment slack*/ - kBarrierBytes;
   static constexpr int kStagesRaw = (kBudget - kOutBytes) / kStageBytes;
-  static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
+  static constexpr int kStages = kStagesRaw > 7 ? 7 : kStagesRaw;
   static constexpr int kTotal = kStages * kStageBytes + kOutBytes + kBarrierBytes + 1024;
   static_assert(16 * kStages + 40 + 8 * kGatherSlotsMax <= 256, "barrier area");
   static_assert(kStages >= 2, "the operand pipeline needs at least two stages");
@@ -201,7 +209,7 @@ __device__ __forceinline__ void stage_fp32(uint32_t box, int lane, const float (
 }
 
 template <int BN, int EPI, int NOUT, int CG>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(kThreads<NOUT>, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
             const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmB1,
             const __grid_constant__ CUtensorMap tmOut0, const __grid_constant__ CUtensorMap tmOut1,
@@ -269,7 +277,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_tfull + 8 * s, 1);
-      mbar_init(bar_tempty + 8 * s, kNumEpiWarps * CG);
+      mbar_init(bar_tempty + 8 * s, kEpiWarps<NOUT> * CG);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -629,16 +637,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
   } else {
     // ------------------------------ epilogue ------------------------------
     if constexpr (NOUT == 4) {
-      // TMA-fed mask epilogue (EPI_MASK_FWD / EPI_MASK_BWD on dense sites). Unit = one 64-column box of this
+      // TMA-fed mask epilogue (EPI_MASK_FWD / EPI_MASK_BWD on dense sites). Unit = one 32-column box of this
       // warp's 32 rows; ring of two slots, slot = {box_a: ci in, A / dH out; box_b: H in (bwd), dci or H out}.
       static_assert(EPI == EPI_MASK_FWD || EPI == EPI_MASK_BWD, "TMA-fed epilogue is for the mask epilogues");
       const int ew = warp - 2, q = warp & 3, grp = ew >> 2;
-      const uint32_t ring = smem_out + ew * (4 * kOutBoxBytes);
+      const uint32_t ring = smem_out + ew * (4 * kFedBoxBytes);
       const uint32_t bar_in = smem_bar + 256 + ew * 16;
       constexpr bool kBwd = (EPI == EPI_MASK_BWD);
       const bool want_h = kBwd && args.dci != nullptr;           // H comes in, the mask gradient goes out
       const bool h_out = !kBwd && args.has_out1;                  // forward: H goes out through box_b
-      const uint32_t in_bytes = kOutBoxBytes * (want_h ? 2 : 1);
+      const uint32_t in_bytes = kFedBoxBytes * (want_h ? 2 : 1);
       unsigned long long philox_seed = args.seed;
       if (args.seed_dev != nullptr) philox_seed = *args.seed_dev;
       if (lane == 0) {
@@ -647,7 +655,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         mbar_fence_init();
       }
       __syncwarp();
-      constexpr int nboxes = BN / 64;
+      constexpr int nboxes = BN / 32, kWarpsPerRow = kEpiWarps<NOUT> / 4;
       auto tile_is_real = [&](long long t) {
         if (!args.bgroup_of_mblock) return true;
         int b2, mb2, nb2, sp2;
@@ -664,7 +672,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         while (t < num_tiles) {
           int b2, mb2, nb2, sp2;
           decode(t, b2, mb2, nb2, sp2);
-          if (nb2 * BN + grp * 64 < args.N) break;
+          if (nb2 * BN + grp * 32 < args.N) break;
           t = next_real_tile(t + tstride);
         }
         return t;
@@ -675,14 +683,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         int b2 = 0, mb2 = 0, nb2 = 0, sp2 = 0;
         const bool real = t < num_tiles;  // past the last tile only the wait remains
         if (real) decode(t, b2, mb2, nb2, sp2);
-        const int crow = mb2 * BM + q * 32, col0 = nb2 * BN + j * 64;
-        const uint32_t bar = bar_in + 8 * slot, box_a = ring + slot * (2 * kOutBoxBytes);
-        if (elect_one_sync()) {
+        const int crow = mb2 * BM + q * 32, col0 = nb2 * BN + j * 32;
+        const uint32_t bar = bar_in + 8 * slot, box_a = ring + slot * (2 * kFedBoxBytes);
+        if (lane == 0) {  // the lane that issues the stores: bulk groups are counted per thread
           if (after_stores) tma_store_wait_read<0>();
           if (real) {
             mbar_expect_tx(bar, in_bytes);
             tma_load_3d(box_a, &tmCi, bar, col0, crow, 0);
-            if (want_h) tma_load_3d(box_a + kOutBoxBytes, &tmH, bar, col0, crow, 0);
+            if (want_h) tma_load_3d(box_a + kFedBoxBytes, &tmH, bar, col0, crow, 0);
           }
         }
       };
@@ -712,11 +720,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         if (args.timeline != nullptr && warp == 2 && lane == 0 && unit < 16) stamp(240 + static_cast<int>(unit >> 1));
         const long long t_next = first_unit_from(t + tstride);  // the tile whose first unit follows this tile's last
 #pragma unroll 1
-        for (int j = grp; j < nboxes && !failed; j += 2) {
-          const int col0 = nb * BN + j * 64;
+        for (int j = grp; j < nboxes && !failed; j += kWarpsPerRow) {
+          const int col0 = nb * BN + j * 32;
           if (col0 >= args.N) break;  // uniform across the warp
           const int slot = unit & 1;
-          const uint32_t box_a = ring + slot * (2 * kOutBoxBytes), box_b = box_a + kOutBoxBytes;
+          const uint32_t box_a = ring + slot * (2 * kFedBoxBytes), box_b = box_a + kFedBoxBytes;
           if (!mbar_wait(bar_in + 8 * slot, (unit >> 1) & 1, abort_flag)) {
             if (args.status && lane == 0) atomicCAS(args.status, 0, kTimeoutEpilogue);
             failed = true;
@@ -735,18 +743,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
           }
           if (tl_on) stamp(177 + 8 * static_cast<int>(unit));  // accumulator ready
           const f32x2 rs2 = pk2(rs, rs), ndelta2 = pk2(-delta, -delta), one2 = pk2(1.0f, 1.0f), neg2 = pk2(-1.0f, -1.0f);
-          // One half (32 columns) of the unit: all shared-memory loads first, then the arithmetic of the four
-          // 8-column groups as plain code (four independent Philox chains the scheduler can interleave), then all
+          // One half (16 columns) of the unit: all shared-memory loads first, then the arithmetic of the two
+          // 8-column groups as plain code (two independent Philox chains the scheduler can interleave), then all
           // stores. The loads and stores are `asm volatile` (they must stay behind the barrier waits), so they
           // are kept in two blocks instead of fencing each group's arithmetic from the next.
           auto do_half = [&](const int half) {
-            const int c0 = col0 + 32 * half;
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_row + j * 64 + 32 * half, r);
-            uint4 ciq[4], hq[4];
+            const int c0 = col0 + 16 * half;
+            uint32_t r[16];
+            tmem_ld_16(tmem_row + j * 32 + 16 * half, r);
+            uint4 ciq[2], hq[2];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const uint32_t off = lane * 128 + (((half * 4 + g) ^ (lane & 7)) << 4);
+            for (int g = 0; g < 2; ++g) {
+              const uint32_t off = lane * 64 + (((half * 2 + g) ^ ((lane >> 1) & 3)) << 4);
               asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                            : "=r"(ciq[g].x), "=r"(ciq[g].y), "=r"(ciq[g].z), "=r"(ciq[g].w) : "r"(box_a + off) : "memory");
               hq[g] = make_uint4(0u, 0u, 0u, 0u);
@@ -755,9 +763,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
                              : "=r"(hq[g].x), "=r"(hq[g].y), "=r"(hq[g].z), "=r"(hq[g].w) : "r"(box_b + off) : "memory");
             }
             tmem_ld_wait();
-            uint32_t out_a[4][4], out_b[4][4];
+            uint32_t out_a[2][4], out_b[2][4];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
+            for (int g = 0; g < 2; ++g) {
               const uint32_t ciw[4] = {ciq[g].x, ciq[g].y, ciq[g].z, ciq[g].w}, hw[4] = {hq[g].x, hq[g].y, hq[g].z, hq[g].w};
               f32x2 v2[4], coef2[4], dmdci2[4];
 #pragma unroll
@@ -794,8 +802,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
               }
             }
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const uint32_t off = lane * 128 + (((half * 4 + g) ^ (lane & 7)) << 4);
+            for (int g = 0; g < 2; ++g) {
+              const uint32_t off = lane * 64 + (((half * 2 + g) ^ ((lane >> 1) & 3)) << 4);
               if (kBwd ? want_h : h_out)  // box_b: the mask gradient replaces H (backward), or H goes out (forward)
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(box_b + off), "r"(out_b[g][0]),
                              "r"(out_b[g][1]), "r"(out_b[g][2]), "r"(out_b[g][3]) : "memory");
@@ -810,8 +818,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
             // The other slot's boxes were handed to TMA stores one unit ago: once those have been read,
             // request the NEXT unit's operands into it (they land while this unit's second half is computed).
             long long tn = t;
-            int jn = j + 2;
-            if (!(jn < nboxes && nb * BN + jn * 64 < args.N)) {
+            int jn = j + kWarpsPerRow;
+            if (!(jn < nboxes && nb * BN + jn * 32 < args.N)) {
               tn = t_next;
               jn = grp;
             }
@@ -855,7 +863,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
           acc_phase ^= 1;
         }
       }
-      if (lane == 0) tma_store_wait_all<0>();
+      if (lane == 0) tma_store_wait_read<0>();  // the kernel's end makes the writes visible
     } else {
     // Work unit = a 32-column half of an output box. Global operands of the mask epilogues
     // (ci / W rows, and H rows in the backward) are requested one unit ahead, across box and tile
@@ -1175,7 +1183,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
       for (int o = 16; o > 0; o >>= 1) faith_acc += __shfl_xor_sync(0xffffffffu, faith_acc, o);
       if (lane == 0 && args.dci != nullptr) atomicAdd(args.dci, faith_acc);
     }
-    if (lane == 0) tma_store_wait_all<0>();
+    if (lane == 0) {
+      // The boxes must have been read before the shared memory goes away; the kernel's end makes local writes
+      // visible. Reductions into peers' buffers are waited for in full.
+      if (args.rs_world > 1)
+        tma_store_wait_all<0>();
+      else
+        tma_store_wait_read<0>();
+    }
     }  // NOUT != 4
   }
 
@@ -1271,7 +1286,7 @@ static int launch_gemm(const CUtensorMap& a0, const CUtensorMap& b0, const CUten
   if constexpr (CG == 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kNumThreads);
+    cfg.blockDim = dim3(kThreads<NOUT>);
     cfg.dynamicSmemBytes = Plan::kTotal;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1284,7 +1299,7 @@ static int launch_gemm(const CUtensorMap& a0, const CUtensorMap& b0, const CUten
     cudaError_t le = cudaLaunchKernelEx(&cfg, kern, a0, b0, a1, b1, o0, o1, mci, mh, mdci, peers, launch_args);
     return le == cudaSuccess ? 0 : 400 + static_cast<int>(le);
   }
-  kern<<<grid, kNumThreads, Plan::kTotal, stream>>>(a0, b0, a1, b1, o0, o1, mci, mh, mdci, peers, launch_args);
+  kern<<<grid, kThreads<NOUT>, Plan::kTotal, stream>>>(a0, b0, a1, b1, o0, o1, mci, mh, mdci, peers, launch_args);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + static_cast<int>(e);
 }
@@ -1339,13 +1354,40 @@ struct PdGemmCall {
   int epi_tma;  // mask epilogues: 0 = TMA-fed form where the call allows it and K is short, 1 = never, 2 = whenever allowed
 };
 
+// Tile of a product that leaves the choice open (bn = 0, cta_group = 0): the narrowest one whose tiles still fit one wave.
+// A CTA's time is set-up and first load (about 3 us), its K loop, and the epilogue of its columns, so while SMs are idle
+// narrower tiles on more SMs end sooner; past one wave the 256 x 256 tile of a CTA pair moves the fewest operand bytes.
+// Measured (us, pair 256 / single 256 / 128 / 64 columns): 512 x 256 x 256 8.4 / 7.5 / 6.1 / 5.8; 2048 x 768 x 768
+// 11.1 / 10.2 / 8.9 / 12.5 (64 takes two waves); 4096 x 768 x 768 11.4 / 10.4 / 13.6 / 16.7; 4096 x 768 x 8192
+// 46.6 / 55.2 / 86 / 123: a single CTA re-reads more per K block, which a long K loop pays for (27.2 against 28.1 at
+// K = 4096). Mask products 4096 x 512 x 768: 14.9 / 15.3 / 11.4; a wider mask product stays on pairs.
+static void choose_tile(const PdGemmCall& c, int& bn, int& single_cta) {
+  bn = c.bn == 128 || c.bn == 64 ? c.bn : 256;
+  single_cta = c.cta_group == 1;
+  if (c.bn != 0 || c.cta_group != 0 || c.max_ctas != 0 || c.bgroup_of_mblock != nullptr || c.kblock_range != nullptr ||
+      c.ag_world > 1 || c.rs_world > 1)
+    return;
+  constexpr long long kSms = 148;
+  const long long rows = static_cast<long long>((c.M + BM - 1) / BM) * c.batch * (c.split_k > 1 ? c.split_k : 1);
+  auto one_wave = [&](int n) { return rows * ((c.N + n - 1) / n) <= kSms; };
+  const bool mask = c.epi == EPI_MASK_FWD || c.epi == EPI_MASK_BWD;
+  if (!mask && one_wave(64))
+    bn = 64;
+  else if (one_wave(128))
+    bn = 128;
+  else if (!mask && one_wave(256) && c.K0 + c.K1 <= 4096)
+    single_cta = 1;
+}
+
 extern "C" int pd_gemm(const PdGemmCall* c, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   if (c->M <= 0 || c->N <= 0 || c->batch <= 0 || c->K0 <= 0) return kBadArgument;
   if (c->epi != EPI_PLAIN && (c->batch != 1 || c->accumulate || c->out_fp32)) return kBadArgument;
   if (c->accumulate && !c->out_fp32) return kBadArgument;
-  const int bn = c->bn == 128 ? 128 : 256;
+  if (c->bn == 64 && c->epi != EPI_PLAIN && c->epi != EPI_FAITH) return kBadArgument;
   const int nout = (c->epi == EPI_MASK_FWD && c->out1 != nullptr) ? 2 : 1;
+  int bn, single_cta;
+  choose_tile(*c, bn, single_cta);
 
   GemmArgs a{};
   a.M = c->M; a.N = c->N; a.batch = c->batch;
@@ -1426,7 +1468,7 @@ extern "C" int pd_gemm(const PdGemmCall* c, void* stream_v) {
                        c->M >= 2 * BM && (c->max_ctas == 0 || c->max_ctas >= 2);
   // Pairs halve each CTA's share of the B tile (less shared-memory fill per MMA) and win on every flagship
   // shape measured, K-major or MN-major operands alike.
-  const bool pair = pair_ok && c->cta_group != 1 && (c->cta_group == 2 || g_pair_default);
+  const bool pair = pair_ok && !single_cta && (c->cta_group == 2 || g_pair_default);
   const int b_box = pair ? bn / 2 : bn;
   if ((rc = encode_operand(&ta0, A0, c->M, c->K0, a_batch, BM))) return 1000 + rc;
   if ((rc = encode_operand(&tb0, B0, c->N, c->K0, b_batch, b_box))) return 2000 + rc;
@@ -1454,18 +1496,23 @@ extern "C" int pd_gemm(const PdGemmCall* c, void* stream_v) {
   // ring would take, so the automatic choice keeps it to short K.
   CUtensorMap tci = to0, th = to0, tdci = to0;
   bool epi_tma = false;
-  if ((c->epi == EPI_MASK_FWD || c->epi == EPI_MASK_BWD) && c->epi_tma != 1 && bn == 256 && c->rowmap == nullptr &&
+  if ((c->epi == EPI_MASK_FWD || c->epi == EPI_MASK_BWD) && c->epi_tma != 1 && c->rowmap == nullptr &&
       c->bgroup_of_mblock == nullptr && c->ag_world <= 1 && c->rs_world <= 1 && c->ld_ci >= c->N &&
       (c->epi_tma == 2 || c->K0 + c->K1 <= 1536)) {
     const bool want_h = c->epi == EPI_MASK_BWD && c->dci != nullptr;
     epi_tma = !(want_h && (!c->dci_bf16 || c->dci_accumulate || c->ld_h < c->N || c->ld_dci < c->N));
     if (epi_tma) {
-      if ((rc = encode_tmap(&tci, c->ci, 2, false, c->N, c->M, c->ld_ci, 1, 0, 64, 32))) return 8000 + rc;
+      if ((rc = encode_tmap(&tci, c->ci, 2, false, c->N, c->M, c->ld_ci, 1, 0, 32, 32))) return 8000 + rc;
       if (want_h) {
-        if ((rc = encode_tmap(&th, c->H, 2, false, c->N, c->M, c->ld_h, 1, 0, 64, 32))) return 8100 + rc;
-        if ((rc = encode_tmap(&tdci, c->dci, 2, false, c->N, c->M, c->ld_dci, 1, 0, 64, 32))) return 8200 + rc;
+        if ((rc = encode_tmap(&th, c->H, 2, false, c->N, c->M, c->ld_h, 1, 0, 32, 32))) return 8100 + rc;
+        if ((rc = encode_tmap(&tdci, c->dci, 2, false, c->N, c->M, c->ld_dci, 1, 0, 32, 32))) return 8200 + rc;
       }
-      if (c->epi == EPI_MASK_FWD && nout != 2) to1 = to0;
+      if ((rc = encode_tmap(&to0, c->out0, 2, true, c->N, c->M, c->ldo0, 1, 0, 32, 32))) return 5000 + rc;
+      if (nout == 2) {
+        if ((rc = encode_tmap(&to1, c->out1, 2, false, c->N, c->M, c->ldo1, 1, 0, 32, 32))) return 6000 + rc;
+      } else {
+        to1 = to0;
+      }
     }
   }
   for (int r = 0; r < kMaxPeers; ++r) peers.m[r] = to0;
@@ -1479,8 +1526,9 @@ extern "C" int pd_gemm(const PdGemmCall* c, void* stream_v) {
 #define PD_LAUNCH2(EPI_, NOUT_) \
   launch_gemm<256, EPI_, NOUT_, 2>(ta0, tb0, ta1, tb1, to0, to1, tci, th, tdci, peers, a, c->max_ctas, stream)
   if (epi_tma) {
-    if (c->epi == EPI_MASK_FWD) return pair ? PD_LAUNCH2(EPI_MASK_FWD, 4) : PD_LAUNCH(256, EPI_MASK_FWD, 4);
-    return pair ? PD_LAUNCH2(EPI_MASK_BWD, 4) : PD_LAUNCH(256, EPI_MASK_BWD, 4);
+    if (c->epi == EPI_MASK_FWD)
+      return pair ? PD_LAUNCH2(EPI_MASK_FWD, 4) : bn == 256 ? PD_LAUNCH(256, EPI_MASK_FWD, 4) : PD_LAUNCH(128, EPI_MASK_FWD, 4);
+    return pair ? PD_LAUNCH2(EPI_MASK_BWD, 4) : bn == 256 ? PD_LAUNCH(256, EPI_MASK_BWD, 4) : PD_LAUNCH(128, EPI_MASK_BWD, 4);
   }
   if (pair) {
     if (c->epi == EPI_PLAIN) return PD_LAUNCH2(EPI_PLAIN, 1);
@@ -1488,13 +1536,15 @@ extern "C" int pd_gemm(const PdGemmCall* c, void* stream_v) {
     if (c->epi == EPI_MASK_BWD) return PD_LAUNCH2(EPI_MASK_BWD, 1);
     if (c->epi == EPI_FAITH) return PD_LAUNCH2(EPI_FAITH, 1);
   }
-  if (c->epi == EPI_PLAIN) return bn == 256 ? PD_LAUNCH(256, EPI_PLAIN, 1) : PD_LAUNCH(128, EPI_PLAIN, 1);
+  if (c->epi == EPI_PLAIN)
+    return bn == 256 ? PD_LAUNCH(256, EPI_PLAIN, 1) : bn == 128 ? PD_LAUNCH(128, EPI_PLAIN, 1) : PD_LAUNCH(64, EPI_PLAIN, 1);
   if (c->epi == EPI_MASK_FWD) {
     if (nout == 2) return bn == 256 ? PD_LAUNCH(256, EPI_MASK_FWD, 2) : PD_LAUNCH(128, EPI_MASK_FWD, 2);
     return bn == 256 ? PD_LAUNCH(256, EPI_MASK_FWD, 1) : PD_LAUNCH(128, EPI_MASK_FWD, 1);
   }
   if (c->epi == EPI_MASK_BWD) return bn == 256 ? PD_LAUNCH(256, EPI_MASK_BWD, 1) : PD_LAUNCH(128, EPI_MASK_BWD, 1);
-  if (c->epi == EPI_FAITH) return bn == 256 ? PD_LAUNCH(256, EPI_FAITH, 1) : PD_LAUNCH(128, EPI_FAITH, 1);
+  if (c->epi == EPI_FAITH)
+    return bn == 256 ? PD_LAUNCH(256, EPI_FAITH, 1) : bn == 128 ? PD_LAUNCH(128, EPI_FAITH, 1) : PD_LAUNCH(64, EPI_FAITH, 1);
 #undef PD_LAUNCH2
 #undef PD_LAUNCH
   return kBadArgument;

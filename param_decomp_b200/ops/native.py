@@ -167,7 +167,7 @@ def gemm(
     bias: torch.Tensor | None = None,
     act: str | None = None,
     split_k: int = 1,
-    bn: int = 256,
+    bn: int = 0,  # tile columns 64 / 128 / 256; 0 = chosen by size (with cta_group = 0)
     epi: int = EPI_PLAIN,
     out1: torch.Tensor | None = None,
     ci: torch.Tensor | None = None,

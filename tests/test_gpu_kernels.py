@@ -977,3 +977,23 @@ def test_flash_attention_walks_items(nv, hd, T, H, Hkv, B):
         ref = ports.sdpa_reference(q.float(), k.float(), v.float(), causal, None)
         _done(nv)
         assert rel(out, ref) < 6e-3, (causal, rel(out, ref))  # bf16 probabilities and outputs: 2^-8 each
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 65, 72), (512, 256, 256), (1160, 1030, 136), (2048, 768, 192), (2304, 1040, 64),
+                                   (4096, 768, 128), (4736, 1024, 64), (4096, 1096, 4104)])
+def test_gemm_tile_choice_by_size(nv, M, N, K):
+    """Both sides of every line of the automatic choice (64, 128, 256 columns on one CTA, CTA pairs), with ragged last
+    tiles; the choice never changes an element's sum order, so all forms agree with fp32 to bf16 rounding."""
+    torch.manual_seed(M + N)
+    N8 = (N + 7) // 8 * 8
+    a, b = torch.randn(M, K, device="cuda", dtype=bf), torch.randn(N, K, device="cuda", dtype=bf)
+    out = torch.zeros(M, N8, device="cuda", dtype=bf)[:, :N]
+    nv.gemm(a, b, out)
+    ref = a.float() @ b.float().T
+    at, acc = a.T.contiguous() if M % 8 == 0 else None, torch.zeros(M, (N + 3) // 4 * 4, device="cuda")[:, :N]
+    if at is not None:
+        nv.gemm(at, b, acc, a_mn=True, accumulate=True, split_k=2)
+    _done(nv)
+    assert rel(out, ref) < 2**-8
+    if at is not None:
+        assert rel(acc, ref) < 1e-5
