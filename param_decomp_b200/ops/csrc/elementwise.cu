@@ -302,23 +302,29 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gate,
   }
 }
 
-// y[row, :] = x[row, :] * s[row]
+// y[row, :] = x[row, :] * s[row], a warp per row: no division per piece, the scale is read once a row. 32768 x 768 bf16
+// (100 MB): 19 us either way; 4096 x 768 .. 3072: 9.2 us on
+// average with a 64-bit division per 16 bytes, 7.2 us now.
 __global__ void rowscale_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s,
                                 __nv_bfloat16* __restrict__ y, long long rows, int d) {
-  const long long total = rows * (d / 8);
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long row = i / (d / 8);
+  const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+  for (long long row = static_cast<long long>(blockIdx.x) * warps + (threadIdx.x >> 5); row < rows;
+       row += static_cast<long long>(gridDim.x) * warps) {
     const float sc = s[row];
-    const uint4 q = *reinterpret_cast<const uint4*>(x + i * 8);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-    __nv_bfloat162 o[4];
+    const __nv_bfloat16* xr = x + row * d;
+    __nv_bfloat16* yr = y + row * d;
+#pragma unroll 4
+    for (int i = lane * 8; i < d; i += 256) {
+      const uint4 q = *reinterpret_cast<const uint4*>(xr + i);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+      __nv_bfloat162 o[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 f = __bfloat1622float2(h[k]);
-      o[k] = __floats2bfloat162_rn(f.x * sc, f.y * sc);
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = __bfloat1622float2(h[k]);
+        o[k] = __floats2bfloat162_rn(f.x * sc, f.y * sc);
+      }
+      *reinterpret_cast<uint4*>(yr + i) = *reinterpret_cast<uint4*>(o);
     }
-    *reinterpret_cast<uint4*>(y + i * 8) = *reinterpret_cast<uint4*>(o);
   }
 }
 
@@ -432,23 +438,33 @@ __global__ void ci_squash_activity_kernel(const __nv_bfloat16* __restrict__ pre,
   const int col = (blockIdx.x * 32 + cg) * 8;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (col < C) {
-    for (long long r = static_cast<long long>(blockIdx.y) * 8 + rl; r < rows;
-         r += static_cast<long long>(gridDim.y) * 8) {
-      const uint4 q = *reinterpret_cast<const uint4*>(pre + r * C + col);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-      __nv_bfloat162 lo[4];
+    const long long stride = static_cast<long long>(gridDim.y) * 8;
+    auto one = [&](long long r, const uint4& q) {
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+      uint32_t lo[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float2 f = __bfloat1622float2(h[k]);
+        const float2 f = pd::unpack2(pd::unpack_bf16_2(w[k]));
         const float lx = fminf(fmaxf(f.x, 0.f), 1.f), ly = fminf(fmaxf(f.y, 0.f), 1.f);
-        lo[k] = __floats2bfloat162_rn(lx, ly);
+        lo[k] = pd::pack_bf16_2(pd::pk2(lx, ly));
         const float ux = f.x > 1.f ? 1.f + alpha * (f.x - 1.f) : lx;
         const float uy = f.y > 1.f ? 1.f + alpha * (f.y - 1.f) : ly;
-        acc[2 * k] += norm * __fdividef(ux * ux, ux * ux + gamma2);
-        acc[2 * k + 1] += norm * __fdividef(uy * uy, uy * uy + gamma2);
+        acc[2 * k] += __fdividef(ux * ux, ux * ux + gamma2);
+        acc[2 * k + 1] += __fdividef(uy * uy, uy * uy + gamma2);
       }
-      *reinterpret_cast<uint4*>(lower + r * C + col) = *reinterpret_cast<uint4*>(lo);
+      *reinterpret_cast<uint4*>(lower + r * C + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    };
+    long long r = static_cast<long long>(blockIdx.y) * 8 + rl;
+    for (; r + 3 * stride < rows; r += 4 * stride) {  // four rows in flight
+      uint4 q[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) q[j] = *reinterpret_cast<const uint4*>(pre + (r + j * stride) * C + col);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) one(r + j * stride, q[j]);
     }
+    for (; r < rows; r += stride) one(r, *reinterpret_cast<const uint4*>(pre + r * C + col));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[k] *= norm;
   }
   __shared__ float red[8][32][8];
 #pragma unroll
@@ -778,9 +794,9 @@ __global__ void colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, float* _
   const int col = (blockIdx.x * 32 + cg) * 8;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (col < C) {
-    for (long long r = static_cast<long long>(blockIdx.y) * 8 + rl; r < rows;
-         r += static_cast<long long>(gridDim.y) * 8) {
-      const uint4 q = *reinterpret_cast<const uint4*>(x + r * C + col);
+    const long long stride = static_cast<long long>(gridDim.y) * 8;
+    long long r = static_cast<long long>(blockIdx.y) * 8 + rl;
+    auto add = [&](const uint4& q) {
       const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -788,7 +804,15 @@ __global__ void colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, float* _
         acc[2 * k] += f.x;
         acc[2 * k + 1] += f.y;
       }
+    };
+    for (; r + 7 * stride < rows; r += 8 * stride) {  // eight rows in flight
+      uint4 q[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) q[j] = *reinterpret_cast<const uint4*>(x + (r + j * stride) * C + col);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) add(q[j]);
     }
+    for (; r < rows; r += stride) add(*reinterpret_cast<const uint4*>(x + r * C + col));
   }
   __shared__ float red[8][32][8];
 #pragma unroll
@@ -806,6 +830,15 @@ __global__ void colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, float* _
 }
 
 }  // namespace
+
+// Row chunks of the column reductions (256 columns a block, one atomic per column and chunk): enough blocks for four per
+// SM, but at least 64 rows each - the chunks of a column add to one address, one after the other. 4096 x 512 .. 1024:
+// 19.5 us on average with 16 rows a chunk, 8.4 us now; the squash over 4096 x 1024 15.7 -> 11.3 us.
+static int column_chunks(long long rows, int gx) {
+  long long gy = (148 * 4 + gx - 1) / gx;
+  if (gy > (rows + 63) / 64) gy = (rows + 63) / 64;
+  return static_cast<int>(gy < 1 ? 1 : gy);
+}
 
 #define PD_CHECK_LAUNCH() (cudaGetLastError() == cudaSuccess ? 0 : 1)
 
@@ -897,7 +930,7 @@ extern "C" int pd_swiglu_bwd(const void* gate, const void* up, const void* dout,
 }
 extern "C" int pd_rowscale(const void* x, const float* s, void* y, long long rows, int d, void* stream) {
   if (d % 8 != 0) return 5;
-  rowscale_kernel<<<blocks_for(rows * (d / 8), kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  rowscale_kernel<<<blocks_for(rows, kThreads / 32), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), s, static_cast<__nv_bfloat16*>(y), rows, d);
   return PD_CHECK_LAUNCH();
 }
@@ -928,10 +961,7 @@ extern "C" int pd_ci_squash_activity(const void* pre, void* lower, float* colsum
                                      float gamma, int normalize_at_one, float alpha, const float* gamma_dev,
                                      void* stream) {
   if (C % 8 != 0) return 5;
-  const int gx = (C + 255) / 256;
-  int gy = (148 * 4 + gx - 1) / gx;
-  if (gy > (rows + 7) / 8) gy = static_cast<int>((rows + 7) / 8);
-  if (gy < 1) gy = 1;
+  const int gx = (C + 255) / 256, gy = column_chunks(rows, gx);
   const float g2 = gamma * gamma;
   ci_squash_activity_kernel<<<dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(pre), static_cast<__nv_bfloat16*>(lower), colsum, rows, C, g2,
@@ -1002,10 +1032,7 @@ extern "C" int pd_split3_bf16(const float* x, void* out, long long g, long long 
 
 extern "C" int pd_colsum_bf16(const void* x, float* out, long long rows, int C, void* stream) {
   if (C % 8 != 0) return 5;
-  const int gx = (C + 255) / 256;
-  int gy = (148 * 4 + gx - 1) / gx;
-  if (gy > (rows + 7) / 8) gy = static_cast<int>((rows + 7) / 8);
-  if (gy < 1) gy = 1;
+  const int gx = (C + 255) / 256, gy = column_chunks(rows, gx);
   colsum_bf16_kernel<<<dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), out, rows, C);
   return PD_CHECK_LAUNCH();

@@ -997,3 +997,23 @@ def test_gemm_tile_choice_by_size(nv, M, N, K):
     assert rel(out, ref) < 2**-8
     if at is not None:
         assert rel(acc, ref) < 1e-5
+
+
+@pytest.mark.parametrize("rows,C", [(1, 8), (63, 264), (4096, 512), (5000, 1032)])
+def test_column_reductions_and_rowscale_edges(nv, rows, C):
+    """Remainders of the rows held in flight and of the 256-column blocks."""
+    from param_decomp_b200.ops import elementwise as ew
+
+    torch.manual_seed(rows)
+    x = (torch.randn(rows, C, device="cuda") * 0.8).to(bf)
+    s = torch.rand(rows, device="cuda")
+    lower, act = ew.squash_activity(x, 0.5, True)
+    total, scaled = ew.colsum_bf16(x), ew.rowscale(x, s)
+    _done(nv)
+    xd = x.double()
+    u = torch.where(xd > 1, 1 + 0.01 * (xd - 1), xd.clamp(0, 1))
+    assert torch.equal(lower, x.clamp(0, 1))
+    assert torch.allclose(act.double(), (1.25 * u * u / (u * u + 0.25)).mean(0), rtol=1e-5, atol=1e-7)
+    # fp32 sums of at most 5000 values below 4: a few hundred roundings of partial sums below 2^9
+    assert torch.allclose(total.double(), xd.sum(0), rtol=1e-5, atol=2e-3)
+    assert torch.equal(scaled, (x.float() * s[:, None]).to(bf))
