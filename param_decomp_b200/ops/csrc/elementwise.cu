@@ -423,11 +423,11 @@ __global__ void ci_squash_kernel(const __nv_bfloat16* __restrict__ pre,
 // ---- fused CI squash + smooth-L0 activity ------------------------------------------------------
 // One pass over the pre-activations [rows, C] (bf16):
 //   lower = clamp(pre, 0, 1)                                   (bf16, feeds the masks)
-//   colsum[c] += sum_rows psi(upper(pre)),  psi(u) = u^2 / (u^2 + gamma^2) (* (1 + gamma^2))
+//   partial[chunk, c] = sum over the chunk's rows of psi(upper(pre)),  psi(u) = u^2 / (u^2 + gamma^2) (* (1 + gamma^2))
 // Block = 32 column groups of 8 columns x 8 row lanes; grid = (C / 256, row chunks).
 __global__ void ci_squash_activity_kernel(const __nv_bfloat16* __restrict__ pre,
                                           __nv_bfloat16* __restrict__ lower,
-                                          float* __restrict__ colsum, long long rows, int C,
+                                          float* __restrict__ partial, long long rows, int C,
                                           float gamma2, float norm, float alpha, const float* __restrict__ gamma_dev, int normalize) {
   if (gamma_dev != nullptr) {  // the schedule's current value lives in device memory (recorded launches)
     const float gm = *gamma_dev;
@@ -476,7 +476,7 @@ __global__ void ci_squash_activity_kernel(const __nv_bfloat16* __restrict__ pre,
       float v = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) v += red[j][cg][k];
-      atomicAdd(colsum + col + k, v);
+      partial[static_cast<long long>(blockIdx.y) * C + col + k] = v;
     }
   }
 }
@@ -787,8 +787,8 @@ __global__ void split3_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* _
   }
 }
 
-// out[c] += sum over rows of x[row, c] (bf16 in, fp32 out). Same tiling as the activity kernel.
-__global__ void colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long rows,
+// partial[chunk, c] = sum over the chunk's rows of x[row, c] (bf16 in, fp32 out). Same tiling as the activity kernel.
+__global__ void colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ partial, long long rows,
                                    int C) {
   const int cg = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int col = (blockIdx.x * 32 + cg) * 8;
@@ -824,17 +824,36 @@ __global__ void colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, float* _
       float v = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) v += red[j][cg][k];
-      atomicAdd(out + col + k, v);
+      partial[static_cast<long long>(blockIdx.y) * C + col + k] = v;
     }
+  }
+}
+
+// out[c] = scale * sum over chunks of partial[chunk, c], in a fixed order: equal inputs give equal bits.
+__global__ void column_total_kernel(const float* __restrict__ partial, float* __restrict__ out, int chunks, int C,
+                                    float scale) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  float acc = 0.f;
+  if (c < C)
+    for (int y = w; y < chunks; y += 8) acc += partial[static_cast<long long>(y) * C + c];
+  red[w][lane] = acc;
+  __syncthreads();
+  if (w == 0 && c < C) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) acc += red[k][lane];
+    out[c] = acc * scale;
   }
 }
 
 }  // namespace
 
-// Row chunks of the column reductions (256 columns a block, one atomic per column and chunk): enough blocks for four per
-// SM, but at least 64 rows each - the chunks of a column add to one address, one after the other. 4096 x 512 .. 1024:
-// 19.5 us on average with 16 rows a chunk, 8.4 us now; the squash over 4096 x 1024 15.7 -> 11.3 us.
-static int column_chunks(long long rows, int gx) {
+// Row chunks of the column reductions (256 columns a block): enough blocks for four per SM, at least 64 rows each. The
+// chunks' sums go to scratch and are added by a second kernel, which takes the place of clearing the output: with
+// atomics, up to 296 chunks added to one address one after the other, in any order. 4096 x 512 .. 1024: 19.5 us on average with
+// atomics and 16 rows a chunk, 6.3 us now (both kernels); the squash over 4096 x 1024 15.7 -> 9.3 us.
+extern "C" int pd_column_chunks(long long rows, int C) {
+  const int gx = (C + 255) / 256;
   long long gy = (148 * 4 + gx - 1) / gx;
   if (gy > (rows + 63) / 64) gy = (rows + 63) / 64;
   return static_cast<int>(gy < 1 ? 1 : gy);
@@ -957,15 +976,18 @@ extern "C" int pd_ci_squash(const void* pre, void* lower, void* upper, long long
   return PD_CHECK_LAUNCH();
 }
 
-extern "C" int pd_ci_squash_activity(const void* pre, void* lower, float* colsum, long long rows, int C,
+// `mean [C]`: mean activity over rows; `partial [pd_column_chunks(rows, C), C]` is scratch
+extern "C" int pd_ci_squash_activity(const void* pre, void* lower, float* mean, float* partial, long long rows, int C,
                                      float gamma, int normalize_at_one, float alpha, const float* gamma_dev,
                                      void* stream) {
   if (C % 8 != 0) return 5;
-  const int gx = (C + 255) / 256, gy = column_chunks(rows, gx);
+  const int gx = (C + 255) / 256, gy = pd_column_chunks(rows, C);
   const float g2 = gamma * gamma;
   ci_squash_activity_kernel<<<dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(pre), static_cast<__nv_bfloat16*>(lower), colsum, rows, C, g2,
+      static_cast<const __nv_bfloat16*>(pre), static_cast<__nv_bfloat16*>(lower), partial, rows, C, g2,
       normalize_at_one ? 1.f + g2 : 1.f, alpha, gamma_dev, normalize_at_one);
+  column_total_kernel<<<(C + 31) / 32, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      partial, mean, gy, C, static_cast<float>(1.0 / static_cast<double>(rows)));
   return PD_CHECK_LAUNCH();
 }
 extern "C" int pd_ci_squash_activity_bwd(const void* pre, const void* dlower, const float* dcol, void* dpre,
@@ -1030,10 +1052,11 @@ extern "C" int pd_split3_bf16(const float* x, void* out, long long g, long long 
   return PD_CHECK_LAUNCH();
 }
 
-extern "C" int pd_colsum_bf16(const void* x, float* out, long long rows, int C, void* stream) {
+extern "C" int pd_colsum_bf16(const void* x, float* out, float* partial, long long rows, int C, void* stream) {
   if (C % 8 != 0) return 5;
-  const int gx = (C + 255) / 256, gy = column_chunks(rows, gx);
+  const int gx = (C + 255) / 256, gy = pd_column_chunks(rows, C);
   colsum_bf16_kernel<<<dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), out, rows, C);
+      static_cast<const __nv_bfloat16*>(x), partial, rows, C);
+  column_total_kernel<<<(C + 31) / 32, 256, 0, static_cast<cudaStream_t>(stream)>>>(partial, out, gy, C, 1.f);
   return PD_CHECK_LAUNCH();
 }

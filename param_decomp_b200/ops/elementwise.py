@@ -181,6 +181,13 @@ def swiglu(gate: Tensor, up: Tensor) -> Tensor:
     return _SwiGLU.apply(gate, up)
 
 
+def _column_scratch(rows: int, cols: int, device) -> Tensor:
+    """Room for the row chunks' sums of a column reduction."""
+    lib = _lib()
+    lib.pd_column_chunks.argtypes = [C.c_longlong, C.c_int]
+    return torch.empty(lib.pd_column_chunks(rows, cols), cols, device=device, dtype=torch.float32)
+
+
 class _SquashActivity(torch.autograd.Function):
     """`pre [rows, C]` bf16 -> (`lower` bf16, `activity [C]` fp32 = mean over rows of the smooth-L0
     penalty of the upper-leaky importance). One read of `pre` in forward, one fused pass in backward
@@ -192,17 +199,19 @@ class _SquashActivity(torch.autograd.Function):
         rows, Cn = pre.shape
         pre = pre.contiguous()
         lower = torch.empty_like(pre)
-        colsum = torch.zeros(Cn, device=pre.device, dtype=torch.float32)
+        mean = torch.empty(Cn, device=pre.device, dtype=torch.float32)
+        partial = _column_scratch(rows, Cn, pre.device)
         lib = _lib()
-        lib.pd_ci_squash_activity.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_float,
-                                              C.c_int, C.c_float, C.c_void_p, C.c_void_p]
+        lib.pd_ci_squash_activity.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_int,
+                                              C.c_float, C.c_int, C.c_float, C.c_void_p, C.c_void_p]
         g_val, g_ptr = _scalar_arg(gamma)
-        _check(lib.pd_ci_squash_activity(pre.data_ptr(), lower.data_ptr(), colsum.data_ptr(), rows, Cn, g_val,
-                                         int(normalize_at_one), alpha, g_ptr, _s()), "ci_squash_activity")
+        _check(lib.pd_ci_squash_activity(pre.data_ptr(), lower.data_ptr(), mean.data_ptr(), partial.data_ptr(), rows, Cn,
+                                         g_val, int(normalize_at_one), alpha, g_ptr, _s()), "ci_squash_activity")
+        nv.count_launch()
         ctx.save_for_backward(pre)
         ctx.cfg = (gamma, normalize_at_one, alpha)
         ctx.mark_non_differentiable()
-        return lower, colsum / rows
+        return lower, mean
 
     @staticmethod
     def backward(ctx, dlower: Tensor | None, dact: Tensor | None):  # type: ignore[override]
@@ -351,9 +360,12 @@ def colsum_bf16(x: Tensor) -> Tensor:
     lead = x.shape[:-2]
     rows, Cn = x.shape[-2], x.shape[-1]
     flat = x.reshape(-1, rows, Cn)
-    out = torch.zeros(flat.shape[0], Cn, device=x.device, dtype=torch.float32)
+    out = torch.empty(flat.shape[0], Cn, device=x.device, dtype=torch.float32)
+    partial = _column_scratch(rows, Cn, x.device)
     lib = _lib()
-    lib.pd_colsum_bf16.argtypes = [C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_void_p]
+    lib.pd_colsum_bf16.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_void_p]
     for i in range(flat.shape[0]):
-        _check(lib.pd_colsum_bf16(flat[i].data_ptr(), out[i].data_ptr(), rows, Cn, _s()), "colsum_bf16")
+        _check(lib.pd_colsum_bf16(flat[i].data_ptr(), out[i].data_ptr(), partial.data_ptr(), rows, Cn, _s()),
+               "colsum_bf16")
+        nv.count_launch()
     return out.reshape(*lead, Cn)
