@@ -23,6 +23,7 @@ enum StatusCode : int {
   kTimeoutMma = 2,
   kTimeoutEpilogue = 3,
   kTimeoutPeerFlag = 4,
+  kBadExpert = 6,  // a job named an expert that does not exist
   kBadArgument = 5,
 };
 

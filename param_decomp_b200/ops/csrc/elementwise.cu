@@ -328,6 +328,117 @@ __global__ void rowscale_kernel(const __nv_bfloat16* __restrict__ x, const float
   }
 }
 
+// ---- routed rows: the sorted and padded job layout ---------------------------------------------------
+// Jobs sorted by expert (stable), every expert's run padded to a multiple of `pad` rows. One block per expert counts its
+// jobs; one per expert then sums the padded counts before its own, walks the jobs again and gives its own their rows in
+// order. `expert [J]`, `pos [J]` = row of a job, `inv [n_rows]` = job of a row or -1, `bgroup [n_rows / 128]` = expert of
+// a row block or -1, `krange [E, 2]` in 64-row K blocks, `counts [E]`. Bound by the latency of the walks' loads and one
+// barrier per 8192 jobs. It replaces about 40 torch kernels: an expert site (8192 tokens, 42 experts, top 8, forward and
+// backward) went from 1147 to 672 us.
+constexpr int kLayoutThreads = 1024;
+
+// jobs per expert, one block each (a shared-memory histogram of all experts in every block serialises on its adds:
+// 35 of 45 us at 65,536 jobs)
+__global__ void __launch_bounds__(kLayoutThreads) job_count_kernel(const long long* __restrict__ expert, int J, int E,
+                                                                   long long* __restrict__ counts,
+                                                                   long long* __restrict__ pos, int* __restrict__ status) {
+  __shared__ int part[kLayoutThreads / 32];
+  const int tid = threadIdx.x, e = blockIdx.x;
+  int n = 0;
+#pragma unroll 8
+  for (int j = tid; j < J; j += kLayoutThreads) {
+    const long long x = expert[j];
+    n += x == e;
+    if (e == 0 && (x < 0 || x >= E)) {  // refused through the status word; the row keeps later gathers in range
+      pos[j] = 0;
+      atomicCAS(status, 0, pd::kBadExpert);
+    }
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((tid & 31) == 0) part[tid >> 5] = n;
+  __syncthreads();
+  if (tid < 32) {
+    n = __reduce_add_sync(0xffffffffu, part[tid]);
+    if (tid == 0) counts[e] = n;
+  }
+}
+
+__global__ void __launch_bounds__(kLayoutThreads) job_layout_kernel(const long long* __restrict__ expert, int J, int E,
+                                                                    int pad, int n_rows,
+                                                                    const long long* __restrict__ counts,
+                                                                    long long* __restrict__ pos, int* __restrict__ inv,
+                                                                    int* __restrict__ bgroup, int* __restrict__ krange) {
+  __shared__ int warp_sum_s[2][32];
+  __shared__ int start_s, end_s;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = blockIdx.x;
+  if (warp == 0) {
+    int before = 0, all = 0;
+    for (int i = lane; i < E; i += 32) {
+      const int p = (static_cast<int>(counts[i]) + pad - 1) / pad * pad;
+      all += p;
+      if (i < e) before += p;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if (lane == 0) {
+      start_s = before;
+      end_s = all;
+    }
+  }
+  __syncthreads();
+  const int start = start_s, mine = static_cast<int>(counts[e]), stop = start + (mine + pad - 1) / pad * pad;
+  if (tid == 0) {
+    krange[2 * e] = start / 64;
+    krange[2 * e + 1] = stop / 64;
+  }
+  for (int i = start / 128 + tid; i < stop / 128; i += kLayoutThreads) bgroup[i] = e;
+  for (int i = start + mine + tid; i < stop; i += kLayoutThreads) inv[i] = -1;
+  if (e == E - 1) {  // rows past the last expert's
+    for (int i = end_s / 128 + tid; i < n_rows / 128; i += kLayoutThreads) bgroup[i] = -1;
+    for (int i = end_s + tid; i < n_rows; i += kLayoutThreads) inv[i] = -1;
+  }
+  // a warp takes kPer * 32 consecutive jobs a round, so that kPer loads are in flight and a barrier serves 8192 jobs
+  constexpr int kPer = 8, kRound = kPer * kLayoutThreads;
+  int base = start;
+  for (int j0 = 0, turn = 0; j0 < J && base < start + mine; j0 += kRound, turn ^= 1) {
+    const int j = j0 + warp * (32 * kPer) + lane;
+    unsigned ball[kPer];
+    int in_warp = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) ball[i] = __ballot_sync(0xffffffffu, j + 32 * i < J && expert[j + 32 * i] == e);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) in_warp += __popc(ball[i]);
+    if (lane == 0) warp_sum_s[turn][warp] = in_warp;
+    __syncthreads();  // the other buffer's readers have passed: it is written again only after the next barrier
+    const int c = warp_sum_s[turn][lane];
+    int total = c, ahead = lane < warp ? c : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      total += __shfl_xor_sync(0xffffffffu, total, o);
+      ahead += __shfl_xor_sync(0xffffffffu, ahead, o);
+    }
+    int row = base + ahead;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (ball[i] >> lane & 1u) {
+        const int at = row + __popc(ball[i] & ((1u << lane) - 1u));
+        pos[j + 32 * i] = at;
+        inv[at] = j + 32 * i;
+      }
+      row += __popc(ball[i]);
+    }
+    base += total;
+  }
+}
+
+// rowmap[row] = (token, first column of the slot) of the row's job; token -1 on padding rows
+__global__ void job_rowmap_kernel(const int* __restrict__ inv, int4* __restrict__ rowmap, int n_rows, int k, int c) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n_rows) return;
+  const int j = inv[r];
+  rowmap[r] = j < 0 ? make_int4(-1, 0, 0, 0) : make_int4(j / k, j % k * c, 0, 0);
+}
+
 // ---- routed rows: tokens <-> padded sorted job rows -----------------------------------------------
 // `rowmap[r] = (token, slot, -, -)` of padded row r (token -1 on padding rows); `pos[token * k + slot]`
 // is the inverse. Both directions move whole rows in 16-byte pieces; no row is written twice, so
@@ -951,6 +1062,20 @@ extern "C" int pd_rowscale(const void* x, const float* s, void* y, long long row
   if (d % 8 != 0) return 5;
   rowscale_kernel<<<blocks_for(rows, kThreads / 32), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), s, static_cast<__nv_bfloat16*>(y), rows, d);
+  return PD_CHECK_LAUNCH();
+}
+extern "C" int pd_job_layout(const long long* expert, int J, int E, int pad, int n_rows, long long* pos, int* inv,
+                             int* bgroup, int* krange, long long* counts, int* status, void* stream) {
+  if (J <= 0 || E <= 0 || E > 8192 || (pad != 128 && pad != 256) || n_rows % 128 != 0) return 5;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  job_count_kernel<<<E, kLayoutThreads, 0, st>>>(expert, J, E, counts, pos, status);
+  job_layout_kernel<<<E, kLayoutThreads, 0, st>>>(expert, J, E, pad, n_rows, counts, pos, inv, bgroup, krange);
+  return PD_CHECK_LAUNCH();
+}
+extern "C" int pd_job_rowmap(const int* inv, void* rowmap, int n_rows, int k, int c, void* stream) {
+  if (n_rows <= 0 || k <= 0) return 5;
+  job_rowmap_kernel<<<(n_rows + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(inv, static_cast<int4*>(rowmap),
+                                                                                      n_rows, k, c);
   return PD_CHECK_LAUNCH();
 }
 extern "C" int pd_rows_expand(const void* x, const void* rowmap, const float* w, void* out, long long n_rows,

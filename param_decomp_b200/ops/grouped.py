@@ -42,6 +42,7 @@ class JobLayout:
     bgroup: Tensor  # [n_rows / 128] int32: expert of each row block, -1 for unused tail blocks
     krange: Tensor  # [E, 2] int32: 64-row K-block range of each expert
     counts: Tensor  # [E] int64
+    inv: Tensor | None = None  # [n_rows] int32: job of each row, -1 on padding rows (when a kernel built the layout)
 
     @classmethod
     def cached(cls, indices: Tensor, n_experts: int) -> "JobLayout":
@@ -84,6 +85,13 @@ class JobLayout:
     @classmethod
     def build(cls, expert_of_job: Tensor, n_experts: int) -> "JobLayout":
         J = expert_of_job.numel()
+        # static upper bound on rows so shapes do not depend on the routing (no host sync)
+        n_rows = (J + n_experts * (PAD - 1) + PAD - 1) // PAD * PAD
+        # Two kernels while their blocks (one per expert, each walking all jobs) are short: at 2^19 jobs a walk is 64
+        # rounds of 8192 jobs; longer lists take the sort below.
+        if expert_of_job.is_cuda and 0 < J <= 1 << 19 and n_experts <= 8192 and expert_of_job.dtype == torch.int64:
+            pos, inv, bgroup, krange, counts = ew.job_layout(expert_of_job.contiguous(), n_experts, PAD, n_rows)
+            return cls(pos, n_rows, bgroup, krange, counts, inv)
         # (a scatter-add, not bincount: bincount sizes its output from the data and synchronises)
         counts = torch.zeros(n_experts, dtype=torch.int64, device=expert_of_job.device).scatter_add_(
             0, expert_of_job, torch.ones_like(expert_of_job))
@@ -95,8 +103,6 @@ class JobLayout:
         rank_in_group = torch.arange(J, device=expert_of_job.device) - first[sorted_e]
         pos = torch.empty(J, dtype=torch.int64, device=expert_of_job.device)
         pos[order] = starts[sorted_e] + rank_in_group
-        # static upper bound on rows so shapes do not depend on the routing (no host sync)
-        n_rows = (J + n_experts * (PAD - 1) + PAD - 1) // PAD * PAD
         blocks = torch.arange(n_rows // BLOCK, device=pos.device) * BLOCK
         ends = starts + padded
         owner = torch.searchsorted(ends, blocks, right=True)
@@ -111,6 +117,8 @@ class JobLayout:
         rows carry token -1."""
         key = (k, c)
         cache = self.__dict__.setdefault("_rowmaps", {})
+        if key not in cache and self.inv is not None:
+            cache[key] = ew.job_rowmap(self.inv, k, c)
         if key not in cache:
             J = self.pos.numel()
             j = torch.arange(J, device=self.pos.device)

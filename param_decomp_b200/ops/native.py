@@ -120,10 +120,12 @@ def _status_ptr(device_index: int) -> int:
 
 
 def check_status() -> None:
-    """Synchronising check of the status word; raises if a bounded wait ran out."""
+    """Synchronising check of the status word; raises if a bounded wait ran out or a kernel refused its input."""
     code = int(status_word().item())
     if code != 0:
         status_word().zero_()
+        if code == 6:
+            raise NativeError("a routed job named an expert outside the bank")
         raise NativeError(f"a device-side wait timed out (status code {code})")
 
 

@@ -1017,3 +1017,20 @@ def test_column_reductions_and_rowscale_edges(nv, rows, C):
     # fp32 sums of at most 5000 values below 4: a few hundred roundings of partial sums below 2^9
     assert torch.allclose(total.double(), xd.sum(0), rtol=1e-5, atol=2e-3)
     assert torch.equal(scaled, (x.float() * s[:, None]).to(bf))
+
+
+@pytest.mark.parametrize("J,E", [(1, 1), (31, 3), (1024, 7), (1025, 64), (5000, 300), (8193, 5), (65536, 42)])
+def test_job_layout_kernel_equals_torch_statement(nv, J, E):
+    """One-launch layout against the sort-based statement (run on the CPU): equal integers, empty experts included."""
+    from param_decomp_b200.ops.grouped import JobLayout
+
+    g = torch.Generator().manual_seed(J)
+    e = torch.randint(0, max(1, E - 1), (J,), generator=g)
+    a, b = JobLayout.build(e.cuda(), E), JobLayout.build(e, E)
+    assert a.inv is not None and b.inv is None and a.n_rows == b.n_rows
+    for f in ("pos", "bgroup", "krange", "counts"):
+        x, y = getattr(a, f), getattr(b, f)
+        assert x.dtype == y.dtype and torch.equal(x.cpu(), y), f
+    for k, c in ((1, 1), (1, 64)) if J % 2 else ((2, 8), (1, 1)):
+        assert torch.equal(a.rowmap(k, c).cpu(), b.rowmap(k, c))
+    _done(nv)
