@@ -63,6 +63,10 @@ struct AttnArgs {
 };
 
 constexpr int kSub = 64;  // keys per softmax step of the forward
+// P V_n reports on barrier n % kOutBars. A parity wait only tells neighbouring phases apart. When a softmax warp waits for
+// P V_n, P V_{n-1} may be running or may have ended, P V_n may have ended too, and nothing later has been issued: with one
+// barrier the state is one of three phases, with two it is "before" or "after".
+constexpr int kOutBars = 2;
 
 template <int HD>
 struct FwdPlan {
@@ -119,10 +123,10 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
   const uint32_t sm_q = base;
   const uint32_t sm_kv = sm_q + Plan::kQBytes;
   const uint32_t sm_bar = sm_kv + kSlots * Plan::kSlotBytes;
-  // barriers: q_full, q_empty, slot_full[8], slot_empty[8], s_full[2], p_full[2], o_full, o_empty
+  // barriers: q_full, q_empty, slot_full[8], slot_empty[8], s_full[2], p_full[2], o_full[2], o_empty
   const uint32_t bar_qf = sm_bar, bar_qe = bar_qf + 8;
   const uint32_t bar_f = bar_qe + 8, bar_e = bar_f + 64, bar_s = bar_e + 64, bar_p = bar_s + 16;
-  const uint32_t bar_o = bar_p + 16, bar_oe = bar_o + 8;
+  const uint32_t bar_o = bar_p + 16, bar_oe = bar_o + 8 * kOutBars;
   const uint32_t tmem_slot = bar_oe + 8;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base));
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
       mbar_init(bar_s + 8 * i, 1);
       mbar_init(bar_p + 8 * i, kSoftmaxThreads);
     }
-    mbar_init(bar_o, 1);
+    for (int i = 0; i < kOutBars; ++i) mbar_init(bar_o + 8 * i, 1);
     mbar_init(bar_oe, kSoftmaxThreads);
     *abort_flag = 0;
     mbar_fence_init();
@@ -160,6 +164,9 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
   const uint32_t tmem_s = *tmem_slot_ptr;
   const uint32_t tmem_o = tmem_s + 2 * kSub;
   const int w0 = static_cast<int>(blockIdx.x), wstep = static_cast<int>(gridDim.x);
+  auto wait_out = [&](uint32_t n) {  // until P V_n has ended
+    return mbar_wait_warp(bar_o + 8 * (n % kOutBars), (n / kOutBars) & 1, abort_flag);
+  };
 
   // Producer and MMA issuer walk one sequence of tensor steps: S_0, S_1, then P V_n, S_{n+2} for every n. Each step
   // takes the next slot of the ring (64 rows of K for S, of V for P V).
@@ -263,12 +270,12 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
         for (int k = 0; k < kSub / 16; ++k)  // 16 keys: eight columns of P, two 8-row groups of V
           umma_bf16_ts(tmem_o, tmem_s + buf * kSub + 8 * k, vd + k * (2048 >> 4), idesc_o, (vc.j > 0 || k > 0) ? 1u : 0u);
         umma_commit(bar_e + 8 * slot);
-        umma_commit(bar_o);
+        umma_commit(bar_o + 8 * (v_count % kOutBars));
       }
       advance_slot();
       vc.advance();
       if (!sc.done()) {  // S_{n+2} overwrites P_n: P V_n has read it
-        ok = mbar_wait_warp(bar_o, v_count & 1, abort_flag);
+        ok = wait_out(v_count);
         if (ok) next_s();
       }
       ++v_count;
@@ -340,7 +347,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
           const float alpha = grow ? fast_exp2(m_ref - m_tile) : 1.0f;  // 0 where nothing was seen before
           if (grow) m_ref = m_tile;
           l2 = mul2(l2, pk2(alpha, alpha));
-          if (!mbar_wait_warp(bar_o, (n - 1) & 1, abort_flag)) { ok = false; break; }
+          if (!wait_out(n - 1)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < HD / 16; ++c) {
@@ -370,8 +377,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
         mbar_arrive(bar_p + 8 * buf);
       }
       if (!ok) break;
-      // both of the last two P V may still run, and a parity only tells neighbouring phases apart: wait for each
-      if (!mbar_wait_warp(bar_o, (n - 2) & 1, abort_flag) || !mbar_wait_warp(bar_o, (n - 1) & 1, abort_flag)) {
+      if (!wait_out(n - 1)) {  // the pipe runs them in order: all of the item's P V have ended
         ok = false;
         break;
       }

@@ -1034,3 +1034,19 @@ def test_job_layout_kernel_equals_torch_statement(nv, J, E):
     for k, c in ((1, 1), (1, 64)) if J % 2 else ((2, 8), (1, 1)):
         assert torch.equal(a.rowmap(k, c).cpu(), b.rowmap(k, c))
     _done(nv)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_flash_attention_shortest_items(nv, hd):
+    """Items of two 64-key steps, several per CTA: every item ends while its last two P V are in flight."""
+    from param_decomp_b200.models import ports
+    from param_decomp_b200.ops import attention as attn
+
+    torch.manual_seed(hd)
+    q, k, v = (torch.randn(70, 128, 12, hd, device="cuda").to(bf) for _ in range(3))  # 840 items, at most 296 CTAs
+    for causal in (True, False):
+        outs = [attn.flash_attention(q, k, v, causal) for _ in range(20)]
+        ref = ports.sdpa_reference(q.float(), k.float(), v.float(), causal, None)
+        _done(nv)
+        assert all(torch.equal(o, outs[0]) for o in outs)
+        assert rel(outs[0], ref) < 6e-3, rel(outs[0], ref)  # bf16 probabilities and outputs: 2^-8 each
