@@ -40,13 +40,17 @@ class SiteWeights:
 
 
 def _split_k_for(M: int, N: int, K: int, sms: int = 148) -> int:
-    """Split count for a weight-gradient GEMM (`K` = tokens): few output tiles leave SMs idle and
-    an unlucky tile count wastes most of its last wave. Up to half a wave of tiles: as many splits as fit one wave
-    (<= 8, >= 128 tokens each; 768 x 1024 over 4096 tokens: 14.9 us with 4, 12.6 us with 6). More tiles: the split
-    (<= 8, >= 1024 tokens per split) whose tile count fills its waves best."""
+    """Split count for a weight-gradient GEMM (`K` = tokens). The splits' fp32 sums are added in no fixed order, so
+    below 2048 tokens the product stays whole and repeatable. From there on few output tiles leave SMs idle and an unlucky
+    tile count wastes most of its last wave. Up to half a wave of tiles: as many splits as fit one wave (<= 8; 768 x 1024
+    over 4096 tokens: 14.9 us with 4, 12.6 us with 6), every one with the same number of 64-token blocks but the last,
+    which may have fewer. More tiles: the split (<= 8, >= 1024 tokens per split) whose tile count fills its waves best."""
+    if K < 2048:
+        return 1
     tiles = ((M + 127) // 128) * ((N + 255) // 256)
     if tiles <= sms // 2:
-        return max(1, min(8, sms // tiles, K // 128))
+        blocks = -(-K // 64)
+        return -(-blocks // -(-blocks // min(8, sms // tiles)))
     best, best_eff = 1, 0.0
     for s in range(1, 9):
         if s > 1 and K // s < 1024:
