@@ -12,12 +12,14 @@
 // S of the next 64 keys is formed while the softmax warps work on the current ones, also across items, so they wait
 // neither for the tensor pipe nor for a new item's first loads. A row's scores are read once into registers; P goes
 // back to tensor memory over the scores it came from, as the A operand of P V, and never touches shared memory. O
-// stays in TMEM and is rescaled only when a row's maximum grows by more than 2^8 over the one its exponents refer to
-// (l, O and the final quotient share that reference, so the result is the same). Tiles off the diagonal of
+// stays in TMEM; a warp rescales its rows there when the maximum of one has grown. The exponents always refer to the
+// running maximum: with an older one as reference (rescaling only past a growth of 2^8) a row's largest probability is a
+// rounded number instead of exactly 1 and the error against 64 bits is 1.5 to 3% larger (forward 93 and 173 us so, 99 and
+// 198 us as it is). Tiles off the diagonal of
 // unsegmented calls take no mask arithmetic. 256 TMEM columns and at most 98 KB a CTA; K and V halves share one ring in the
 // order the tensor pipe takes them. What bounds it is the exponentials (16 lanes a clock: 1024 cycles per 128 x 128).
-// B 64, T 512, 12 heads of 64: 152 us with one 128-key S at a time, P through shared memory and O in registers, 88 us
-// now; B 4, T 2048, 32 / 8 heads of 128: 440 -> 174 us (790 TFLOP/s). One item per CTA and 128 keys a step: 100, 215 us.
+// B 64, T 512, 12 heads of 64: 99 us (152 us with one 128-key S at a time, P through shared memory and O in registers);
+// B 4, T 2048, 32 / 8 heads of 128: 198 us, 695 TFLOP/s (440 us).
 //
 // Backward, one CTA per (128 key rows, kv head, batch), looping over the query heads of the group
 // and the query tiles that see this key tile:
@@ -76,7 +78,6 @@ struct FwdPlan {
   static constexpr int kTotal = kQBytes + kSlots * kSlotBytes + 1024 /*align*/ + 256 /*barriers*/ + 4 * kSub * 4 /*segment ids*/;
   static constexpr uint32_t kTmemCols = 256;            // S / P buffers [0, 64) and [64, 128), O [128, 128 + hd)
 };
-constexpr float kRescaleLog2 = 8.0f;
 
 // The 64-key steps of the items a CTA walks (w, w + stride, ...), in order.
 struct StepCursor {
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
       const int q_idx = sc.qt * kTile + row;
       const int* seg_row = args.segment_ids ? args.segment_ids + static_cast<long long>(sc.b) * args.T : nullptr;
       const int seg_q = seg_row ? seg_row[q_idx] : 0;
-      float m_ref = -INFINITY;  // the maximum the exponents of l and O refer to
+      float m_ref = -INFINITY;  // the row's running maximum, which the exponents of l and O refer to
       f32x2 l2 = 0ull;
       const int diag_j = args.causal ? sc.qt * (kTile / kSub) : 0x7FFFFFFF;  // steps from here on cross the diagonal
       for (int j = 0; j < sc.n_sub; ++j, ++n) {
@@ -340,25 +341,11 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
 #pragma unroll
           for (int c = 0; c < 4; ++c) mx[c] = fmaxf(mx[c], __uint_as_float(r[c >> 1][(c & 1) * 16 + i]));
         const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * args.scale_log2;
-        const bool grow = j == 0 ? m_tile > -INFINITY : m_tile > m_ref + kRescaleLog2;
-        if (j == 0) {
-          if (grow) m_ref = m_tile;
-        } else if (__any_sync(0xffffffffu, grow)) {
-          const float alpha = grow ? fast_exp2(m_ref - m_tile) : 1.0f;  // 0 where nothing was seen before
-          if (grow) m_ref = m_tile;
-          l2 = mul2(l2, pk2(alpha, alpha));
-          if (!wait_out(n - 1)) { ok = false; break; }
-          tc_fence_after();
-#pragma unroll 1
-          for (int c = 0; c < HD / 16; ++c) {
-            uint32_t o[16];
-            tmem_ld_16(tmem_o + lane_base + c * 16, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_16(tmem_o + lane_base + c * 16, o);
-          }
-        }
+        const float m_new = fmaxf(m_ref, m_tile);
+        const float alpha = m_new > m_ref ? fast_exp2(m_ref - m_new) : 1.0f;  // 0 where nothing was seen before
+        const bool rescale = j > 0 && __any_sync(0xffffffffu, m_new > m_ref);
+        m_ref = m_new;
+        l2 = mul2(l2, pk2(alpha, alpha));
         const float m_sub = m_ref == -INFINITY ? 0.0f : -m_ref;  // a row with nothing kept yet: exp2(-inf) = 0
         const f32x2 m2 = pk2(m_sub, m_sub);
 #pragma unroll
@@ -371,6 +358,19 @@ __global__ void __launch_bounds__(kFwdThreads, 2) attn_fwd_kernel(const __grid_c
             l2 = add2(l2, unpack_bf16_2(packed[i]));  // the sum uses the rounded values the tensor core will see
           }
           tmem_st_16(tmem_sp + c * 16, packed);
+        }
+        if (rescale) {  // last, so that P V_{n-1} has run beside the exponentials
+          if (!wait_out(n - 1)) { ok = false; break; }
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < HD / 16; ++c) {
+            uint32_t o[16];
+            tmem_ld_16(tmem_o + lane_base + c * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_16(tmem_o + lane_base + c * 16, o);
+          }
         }
         tmem_st_wait();
         tc_fence_before();
