@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(512) vocab_kl_rows_kernel(const __nv_bfloat16*
   };
   if (tid == 0 && first < rows)
     for (int i = 0; i < pieces; ++i) request(first, i);
+  if (cs > 1) cluster_sync_all();  // every CTA of the cluster runs before another one stores to its shared memory
   const f32x2 l2e = pk2(kLog2E, kLog2E), neg1 = pk2(-1.0f, -1.0f);
   int turn = 0;
   for (long long row = first; row < rows; row += step, ++turn) {
