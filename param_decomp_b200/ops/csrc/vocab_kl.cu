@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(512) vocab_kl_rows_kernel(const __nv_bfloat16*
   }
   __syncthreads();
   const long long first = blockIdx.x / cs, step = gridDim.x / cs;
-  auto request = [&](long long row, int piece) {  // one thread
+  auto request = [&](long long row, int piece) {  // one thread; nothing new once a wait has run out
+    if (*static_cast<volatile int*>(&abort_flag)) return;
     const int g0 = piece * nt, n = min(nt, n_groups - g0);
     const long long at = row * ld + 8ll * (g_first + g0);
     mbar_expect_tx(bar0 + 8 * piece, 32u * n);
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(512) vocab_kl_rows_kernel(const __nv_bfloat16*
         __nv_bfloat16* ta = reinterpret_cast<__nv_bfloat16*>(buf_a + 16 * g);
         __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(buf_b + 16 * g);
         for (int k = 8 - over; k < 8; ++k) ta[k] = tb[k] = __ushort_as_bfloat16(0xFF7Fu);
+        fence_proxy_async_smem();  // before the next row's bulk copy writes here
         a = *reinterpret_cast<const uint4*>(buf_a + 16 * g);
         b = *reinterpret_cast<const uint4*>(buf_b + 16 * g);
       }

@@ -19,3 +19,11 @@ def test_cluster_barrier_before_a_peers_shared_memory(source):
     for name, body in _kernels(CSRC / source).items():
         mapped, barrier = body.find("mapa_shared("), body.find("cluster_sync_all()")
         assert mapped < 0 or 0 <= barrier < mapped, name
+
+
+def test_generic_stores_into_bulk_copy_targets_are_fenced():
+    """vocab_kl writes over the columns past V in a buffer that the next row's bulk copy overwrites: the writing thread's
+    proxy fence follows each such store."""
+    body = _kernels(CSRC / "vocab_kl.cu")["vocab_kl_rows_kernel"]
+    stores = [m.end() for m in re.finditer(r"ta\[k\] = tb\[k\] = [^;]*;", body)]
+    assert stores and all("fence_proxy_async_smem();" in body[at : at + 60] for at in stores)
