@@ -104,7 +104,10 @@ __global__ void vocab_kl_streamed_kernel(const __nv_bfloat16* __restrict__ lc, c
 struct RowSums {
   float ma, mb, sa, sb, cross;  // maxima; sums of exp(a - ma), exp(b - mb), exp(a - ma) (a - b)
 };
-constexpr float kMinMax = -1.0e30f;  // floor of a running maximum: keeps (-inf or lowest) - maximum out of inf - inf
+// Floor of a thread's maximum: a thread that holds only masked logits (-inf or the type's lowest) adds nothing, instead of
+// sums of differences near the end of the range that its zero weight would turn into NaN.
+constexpr float kMinMax = -1.0e30f;
+constexpr float kLowest = -3.3895313892515355e38f;  // lowest finite bf16
 constexpr float kLog2E = 1.4426950408889634f;
 
 __device__ __forceinline__ RowSums merge(const RowSums& x, const RowSums& y) {
@@ -155,6 +158,8 @@ __global__ void __launch_bounds__(512) vocab_kl_rows_kernel(const __nv_bfloat16*
   uint8_t* buf_a = smem;
   uint8_t* buf_b = smem + static_cast<long long>(slice_groups) * 16;
   const uint32_t bar0 = smem_u32(bars);
+  // columns past V in this thread's last group (0 for every thread but the one that holds the row's last group)
+  const int my_over = n_groups > 0 && tid == (n_groups - 1) % nt ? max(0, 8 * (g_first + n_groups) - V) : 0;
   if (tid == 0) {
     for (int i = 0; i < pieces; ++i) mbar_init(bar0 + 8 * i, 1);
     abort_flag = 0;
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(512) vocab_kl_rows_kernel(const __nv_bfloat16*
     for (int i = 0; i < pieces; ++i) request(first, i);
   if (cs > 1) cluster_sync_all();  // every CTA of the cluster runs before another one stores to its shared memory
   const f32x2 l2e = pk2(kLog2E, kLog2E), neg1 = pk2(-1.0f, -1.0f);
-  int turn = 0;
+  int turn = 0, exchange = 0;
   for (long long row = first; row < rows; row += step, ++turn) {
     // this thread's maxima
     uint32_t wa = 0xFF80FF80u, wb = 0xFF80FF80u;  // -inf pairs
@@ -195,55 +200,82 @@ __global__ void __launch_bounds__(512) vocab_kl_rows_kernel(const __nv_bfloat16*
       wa = max_bf16x2(wa, max_bf16x2(max_bf16x2(a.x, a.y), max_bf16x2(a.z, a.w)));
       wb = max_bf16x2(wb, max_bf16x2(max_bf16x2(b.x, b.y), max_bf16x2(b.z, b.w)));
     }
+    const float max_a = fmaxf(__uint_as_float(wa << 16), __uint_as_float(wa & 0xFFFF0000u));
+    const float max_b = fmaxf(__uint_as_float(wb << 16), __uint_as_float(wb & 0xFFFF0000u));
+    // One pass, sums relative to the thread's own maxima. A row whose logits all lie below the floor comes out with a
+    // sum of zero: two more passes, one for the row's true maxima and one for sums relative to them.
     RowSums t;
-    t.ma = fmaxf(kMinMax, fmaxf(__uint_as_float(wa << 16), __uint_as_float(wa & 0xFFFF0000u)));
-    t.mb = fmaxf(kMinMax, fmaxf(__uint_as_float(wb << 16), __uint_as_float(wb & 0xFFFF0000u)));
-    {
-      const f32x2 na = pk2(-t.ma, -t.ma), nb = pk2(-t.mb, -t.mb);
-      f32x2 sa = 0ull, sb = 0ull, cr = 0ull;
-      for (int g = tid; g < n_groups; g += nt) {
-        const uint4 a = *reinterpret_cast<const uint4*>(buf_a + 16 * g), b = *reinterpret_cast<const uint4*>(buf_b + 16 * g);
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+    float ref_a = fmaxf(kMinMax, max_a), ref_b = fmaxf(kMinMax, max_b);
+    for (int pass = 0;; ++pass) {
+      t = RowSums{ref_a, ref_b, 0.0f, 0.0f, 0.0f};
+      if (pass != 1) {
+        const f32x2 na = pk2(-ref_a, -ref_a), nb = pk2(-ref_b, -ref_b);
+        f32x2 sa = 0ull, sb = 0ull, cr = 0ull;
+        for (int g = tid; g < n_groups; g += nt) {
+          const uint4 a = *reinterpret_cast<const uint4*>(buf_a + 16 * g), b = *reinterpret_cast<const uint4*>(buf_b + 16 * g);
+          const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const f32x2 x = unpack_bf16_2(aw[k]), y = unpack_bf16_2(bw[k]);
-          const float2 dx = unpack2(mul2(add2(x, na), l2e)), dy = unpack2(mul2(add2(y, nb), l2e));
-          const f32x2 ea = pk2(ex2(dx.x), ex2(dx.y));
-          sa = add2(sa, ea);
-          sb = add2(sb, pk2(ex2(dy.x), ex2(dy.y)));
-          cr = fma2(ea, fma2(y, neg1, x), cr);
+          for (int k = 0; k < 4; ++k) {
+            const f32x2 x = unpack_bf16_2(aw[k]), y = unpack_bf16_2(bw[k]);
+            const float2 dx = unpack2(mul2(add2(x, na), l2e)), dy = unpack2(mul2(add2(y, nb), l2e));
+            const f32x2 ea = pk2(ex2(dx.x), ex2(dx.y));
+            sa = add2(sa, ea);
+            sb = add2(sb, pk2(ex2(dy.x), ex2(dy.y)));
+            cr = fma2(ea, fma2(y, neg1, x), cr);
+          }
+        }
+        const float2 s0 = unpack2(sa), s1 = unpack2(sb), s2 = unpack2(cr);
+        t.sa = s0.x + s0.y;
+        t.sb = s1.x + s1.y;
+        t.cross = s2.x + s2.y;
+        if (pass == 2 && my_over > 0) {  // the columns past V hold the lowest value, which counts here
+          t.sa -= my_over * ex2((kLowest - ref_a) * kLog2E);
+          t.sb -= my_over * ex2((kLowest - ref_b) * kLog2E);
         }
       }
-      const float2 s0 = unpack2(sa), s1 = unpack2(sb), s2 = unpack2(cr);
-      t.sa = s0.x + s0.y;
-      t.sb = s1.x + s1.y;
-      t.cross = s2.x + s2.y;
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t = merge(t, shuffle_xor(t, o));
-    if (lane == 0) red[warp] = t;
-    __syncthreads();
-    if (warp == 0) {
-      t = red[lane < nt / 32 ? lane : 0];
-      if (lane >= nt / 32) t.sa = t.sb = t.cross = 0.0f;
+      for (int o = 16; o > 0; o >>= 1) t = merge(t, shuffle_xor(t, o));
+      if (lane == 0) red[warp] = t;
+      __syncthreads();
+      if (warp == 0) {
+        t = red[lane < nt / 32 ? lane : 0];
+        if (lane >= nt / 32) t.sa = t.sb = t.cross = 0.0f;
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) t = merge(t, shuffle_xor(t, o));
-      if (lane < cs) {  // to every CTA of the cluster
-        const uint32_t local = smem_u32(&xch[turn & 1][rank]);
-        const uint32_t at = cs > 1 ? mapa_shared(local, lane) : local;
-        store_cluster_f32(at, t.ma);
-        store_cluster_f32(at + 4, t.mb);
-        store_cluster_f32(at + 8, t.sa);
-        store_cluster_f32(at + 12, t.sb);
-        store_cluster_f32(at + 16, t.cross);
+        for (int o = 8; o > 0; o >>= 1) t = merge(t, shuffle_xor(t, o));
+        if (lane < cs) {  // to every CTA of the cluster
+          const uint32_t local = smem_u32(&xch[exchange & 1][rank]);
+          const uint32_t at = cs > 1 ? mapa_shared(local, lane) : local;
+          store_cluster_f32(at, t.ma);
+          store_cluster_f32(at + 4, t.mb);
+          store_cluster_f32(at + 8, t.sa);
+          store_cluster_f32(at + 12, t.sb);
+          store_cluster_f32(at + 16, t.cross);
+        }
+      }
+      if (cs > 1)
+        cluster_sync_all();
+      else
+        __syncthreads();
+      t = xch[exchange & 1][0];
+      for (int r = 1; r < cs; ++r) t = merge(t, xch[exchange & 1][r]);
+      ++exchange;
+      if (pass == 0 && (t.sa == 0.0f || t.sb == 0.0f)) {  // the same verdict in every thread of the cluster
+        ref_a = fmaxf(kLowest, max_a);
+        ref_b = fmaxf(kLowest, max_b);
+      } else if (pass == 1) {
+        ref_a = t.ma;
+        ref_b = t.mb;
+      } else {
+        if (pass == 2 && my_over > 0) {  // and take no part in the gradient
+          const int g = n_groups - 1;
+          __nv_bfloat16* ta = reinterpret_cast<__nv_bfloat16*>(buf_a + 16 * g);
+          __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(buf_b + 16 * g);
+          for (int k = 8 - my_over; k < 8; ++k) ta[k] = tb[k] = __ushort_as_bfloat16(0xFF80u);
+          fence_proxy_async_smem();
+        }
+        break;
       }
     }
-    if (cs > 1)
-      cluster_sync_all();
-    else
-      __syncthreads();
-    t = xch[turn & 1][0];
-    for (int r = 1; r < cs; ++r) t = merge(t, xch[turn & 1][r]);
     // KL = sum p_a (a - lsa - b + lsb) = cross / sa - lsa + lsb
     if (rank == 0 && tid == 0) kl[row] = t.cross / t.sa - (t.ma + __logf(t.sa)) + (t.mb + __logf(t.sb));
     const bool more = row + step < rows;

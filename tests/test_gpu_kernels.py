@@ -1078,3 +1078,34 @@ def test_flash_attention_error_is_that_of_its_roundings(nv, T, hd):
     rounded = (num / den).to(bf).double()
     err = float((out.double().transpose(1, 2) - exact).norm()), float((rounded - exact).norm())
     assert err[0] <= 1.005 * err[1], (err[0] / err[1], err[1] / float(exact.norm()))
+
+
+@pytest.mark.parametrize("V", [1003, 50277, 151936])
+def test_vocab_kl_rows_of_lowest_values(nv, V):
+    """Rows whose logits all lie near the end of the bf16 range in both inputs or in one (uniform distributions), and rows
+    with a single value above the others there; bounds of the sums and of the bf16 gradient as above."""
+    from param_decomp_b200.ops.elementwise import vocab_kl_rows
+
+    torch.manual_seed(V)
+    rows, vp, low = 12, (V + 7) // 8 * 8, torch.finfo(bf).min
+    lc = torch.nn.functional.pad(torch.randn(rows, V, device="cuda").mul_(3).to(bf), (0, vp - V), value=float("nan"))
+    lm = torch.nn.functional.pad(torch.randn(rows, V, device="cuda").mul_(3).to(bf), (0, vp - V), value=float("nan"))
+    dlm_buf = torch.full((rows, vp), float("nan"), device="cuda", dtype=bf)
+    lc, lm = lc[:, :V], lm[:, :V]
+    lc[1], lm[1] = low, low
+    lm[2] = low
+    lc[3] = low
+    lc[4], lm[4] = -2e30, low
+    lc[5], lm[5] = -2e30, -2e30
+    lc[5, V // 2], lm[5, V - 1] = -1.5e30, -1.5e30
+    lc[6], lm[6] = low, low
+    lc[6, 7], lm[6, V - 1] = 0.0, 0.0
+    kl, dlm = vocab_kl_rows(lc, lm, want_grad=True, grad_out=dlm_buf)
+    _done(nv)
+    a, b = (torch.log_softmax(t.double(), -1) for t in (lc, lm))
+    want, d = (a.exp() * (a - b)).sum(-1), b.exp() - a.exp()
+    top = torch.maximum(a, b).exp().amax(-1)
+    assert bool(((dlm.double() - d).abs().amax(-1) <= 2**-8 * top).all())
+    for i in (0, 1, 7, 11):  # finite divergences
+        assert abs(float(kl[i] - want[i])) <= 1e-4 * abs(float(want[i])) + 1e-5, i
+    assert bool((dlm_buf[:, V:] == 0).all())
