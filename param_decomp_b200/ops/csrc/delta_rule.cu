@@ -241,10 +241,13 @@ __global__ void __launch_bounds__(kSerialThreads) delta_bwd_state_kernel(
 //          so the result keeps the accuracy of a direct sum.
 //   dv_t = beta ddelta_t, dbeta_t = ddelta_t . resid_t.
 // Decays are differences of a running sum of g kept in 64 bits (in 32 its rounding would show in D), as are the
-// exponentials and the few hundred final additions of dg.
+// exponentials and the few hundred final additions of dg. A g below -10^4 enters the sum as -10^4: exp of either is 0 in
+// 32 bits, but with -inf the differences past it would be NaN and with -10^18 the later terms of the sum would be lost.
 // 256 threads, a thread owns 4 tokens x DK / 16 columns of dq, dk. Bound by the fp32 FMA rate: 7.3 M FMA per chunk at
 // 128 x 128; the operand tiles take 222 KB of shared memory, one block per SM.
 constexpr int kGradThreads = 256;
+constexpr float kMinLogDecay = -1.0e4f;
+__device__ __forceinline__ double log_decay(float g) { return g < kMinLogDecay ? kMinLogDecay : g; }
 constexpr int kSlice = 16;          // rows of S^T / G^T staged at a time
 constexpr int kWPitch = kChunk + 4;
 
@@ -316,8 +319,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) delta_chunk_grads_kernel(
   const int n = min(kChunk, T - c * kChunk);
 
   if (warp == 0) {  // running sum of g: two tokens per lane
-    const double g0 = 2 * lane < n ? g[row0 + static_cast<long long>(2 * lane) * H] : 0.0f;
-    const double g1 = 2 * lane + 1 < n ? g[row0 + static_cast<long long>(2 * lane + 1) * H] : 0.0f;
+    const double g0 = 2 * lane < n ? log_decay(g[row0 + static_cast<long long>(2 * lane) * H]) : 0.0;
+    const double g1 = 2 * lane + 1 < n ? log_decay(g[row0 + static_cast<long long>(2 * lane + 1) * H]) : 0.0;
     double acc = g0 + g1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

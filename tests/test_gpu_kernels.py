@@ -1109,3 +1109,33 @@ def test_vocab_kl_rows_of_lowest_values(nv, V):
     for i in (0, 1, 7, 11):  # finite divergences
         assert abs(float(kl[i] - want[i])) <= 1e-4 * abs(float(want[i])) + 1e-5, i
     assert bool((dlm_buf[:, V:] == 0).all())
+
+
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64), (32, 32)])
+def test_delta_rule_vanishing_decay(nv, dk, dv):
+    """Decays of one, weak, strong and zero (a log decay of -1e18 and -inf, which forget the state) in one chunk, at its
+    ends and next to each other, against 64 bits; bound as above."""
+    from param_decomp_b200.models import ports
+    from param_decomp_b200.ops import delta_rule
+
+    torch.manual_seed(dk)
+    B, T, H = 2, 140, 2
+    q = ports.l2norm(torch.randn(B, T, H, dk, device="cuda")) * dk**-0.5
+    k = ports.l2norm(torch.randn(B, T, H, dk, device="cuda"))
+    v, beta = torch.randn(B, T, H, dv, device="cuda"), torch.rand(B, T, H, device="cuda")
+    g = -torch.rand(B, T, H, device="cuda")
+    inf = float("inf")
+    for t, x in ((5, -inf), (20, -1e18), (21, 0.0), (22, -inf), (23, -8.0), (40, -300.0), (63, -inf), (64, -1e18), (90, -3e38), (139, -inf)):
+        g[0, t] = x
+    go = torch.randn_like(v)
+    ins = [t.detach().requires_grad_(True) for t in (q, k, v, g, beta)]
+    out = delta_rule.gated_delta_rule(*ins)
+    out.backward(go)
+    ref_ins = [t.detach().double().requires_grad_(True) for t in (q, k, v, g, beta)]
+    ref = ports._delta_rule_sequential(*ref_ins)
+    ref.backward(go.double())
+    _done(nv)
+    for name, a, b in zip("o q k v g beta".split(), [out] + [t.grad for t in ins], [ref] + [t.grad for t in ref_ins]):
+        for i in range(B):  # sequence 0 holds the vanishing decays
+            err = float((a[i].double() - b[i]).norm() / (b[i].norm() + 1e-9))
+            assert err < 3e-6, (name, i, err)
