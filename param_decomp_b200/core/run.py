@@ -377,8 +377,8 @@ def run_decomposition_training(
         keep = cadence.checkpointing.retention.n  # type: ignore[union-attr]
 
     def check_device_status(where: str) -> None:
-        """The native kernels report a wait that ran out (a late or dead peer) in a per-device status word and
-        then run to completion on whatever data they had, so the parameters can no longer be trusted. Read the
+        """The native kernels report a wait that ran out (a late or dead peer) or a refused input (an expert index
+        outside the bank) in a per-device status word and then run to completion on whatever data they had, so the parameters can no longer be trusted. Read the
         word at points where the host waits for the device anyway and stop every rank together, before anything
         is logged as healthy or written to a checkpoint."""
         dev = torch.device(device)
@@ -392,10 +392,10 @@ def run_decomposition_training(
         any_fn = getattr(collectives, "host_any", None)
         bad = bool(any_fn(float(code != 0))) if any_fn is not None else code != 0
         if bad:
-            native.status_word().zero_()
+            native.clear_status()
+            what = native.status_message(code) if code != 0 else "another rank reported a timed-out wait or a refused input"
             raise native.NativeError(
-                f"{where} (step {state.step}): a device-side wait timed out on this or another rank "
-                f"(local status code {code}); the step's results are not valid, stopping without a checkpoint")
+                f"{where} (step {state.step}): {what}; the step's results are not valid, stopping without a checkpoint")
 
     def sync_masters(for_save: bool) -> None:
         """A sharded optimizer keeps each rank's slice of the masters: before anything reads the parameters

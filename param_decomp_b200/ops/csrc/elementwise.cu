@@ -332,28 +332,23 @@ __global__ void rowscale_kernel(const __nv_bfloat16* __restrict__ x, const float
 // Jobs sorted by expert (stable), every expert's run padded to a multiple of `pad` rows. One block per expert counts its
 // jobs; one per expert then sums the padded counts before its own, walks the jobs again and gives its own their rows in
 // order. `expert [J]`, `pos [J]` = row of a job, `inv [n_rows]` = job of a row or -1, `bgroup [n_rows / 128]` = expert of
-// a row block or -1, `krange [E, 2]` in 64-row K blocks, `counts [E]`. Bound by the latency of the walks' loads and one
+// a row block or -1, `krange [E, 2]` in 64-row K blocks, `counts [E]`. A job whose expert does not exist is refused: the
+// status word and `refused` (host memory) say so, and one more block gives such jobs rows of their own past the last
+// expert's, in blocks that no product computes, so that `pos` stays injective and no other job's rows are touched; there
+// is room, since such a job takes one row and `n_rows` counts every job. Bound by the latency of the walks' loads and one
 // barrier per 8192 jobs. It replaces about 40 torch kernels: an expert site (8192 tokens, 42 experts, top 8, forward and
 // backward) went from 1147 to 672 us.
 constexpr int kLayoutThreads = 1024;
 
 // jobs per expert, one block each (a shared-memory histogram of all experts in every block serialises on its adds:
 // 35 of 45 us at 65,536 jobs)
-__global__ void __launch_bounds__(kLayoutThreads) job_count_kernel(const long long* __restrict__ expert, int J, int E,
-                                                                   long long* __restrict__ counts,
-                                                                   long long* __restrict__ pos, int* __restrict__ status) {
+__global__ void __launch_bounds__(kLayoutThreads) job_count_kernel(const long long* __restrict__ expert, int J,
+                                                                   long long* __restrict__ counts) {
   __shared__ int part[kLayoutThreads / 32];
   const int tid = threadIdx.x, e = blockIdx.x;
   int n = 0;
 #pragma unroll 8
-  for (int j = tid; j < J; j += kLayoutThreads) {
-    const long long x = expert[j];
-    n += x == e;
-    if (e == 0 && (x < 0 || x >= E)) {  // refused through the status word; the row keeps later gathers in range
-      pos[j] = 0;
-      atomicCAS(status, 0, pd::kBadExpert);
-    }
-  }
+  for (int j = tid; j < J; j += kLayoutThreads) n += expert[j] == e;
   n = __reduce_add_sync(0xffffffffu, n);
   if ((tid & 31) == 0) part[tid >> 5] = n;
   __syncthreads();
@@ -367,36 +362,41 @@ __global__ void __launch_bounds__(kLayoutThreads) job_layout_kernel(const long l
                                                                     int pad, int n_rows,
                                                                     const long long* __restrict__ counts,
                                                                     long long* __restrict__ pos, int* __restrict__ inv,
-                                                                    int* __restrict__ bgroup, int* __restrict__ krange) {
+                                                                    int* __restrict__ bgroup, int* __restrict__ krange,
+                                                                    int* __restrict__ status, int* __restrict__ refused) {
   __shared__ int warp_sum_s[2][32];
-  __shared__ int start_s, end_s;
+  __shared__ int start_s, known_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, e = blockIdx.x;
   if (warp == 0) {
-    int before = 0, all = 0;
-    for (int i = lane; i < E; i += 32) {
-      const int p = (static_cast<int>(counts[i]) + pad - 1) / pad * pad;
-      all += p;
-      if (i < e) before += p;
+    int before = 0, known = 0;
+    for (int i = lane; i < min(e, E); i += 32) {
+      const int n = static_cast<int>(counts[i]);
+      known += n;
+      before += (n + pad - 1) / pad * pad;
     }
     before = __reduce_add_sync(0xffffffffu, before);
-    all = __reduce_add_sync(0xffffffffu, all);
+    known = __reduce_add_sync(0xffffffffu, known);
     if (lane == 0) {
       start_s = before;
-      end_s = all;
+      known_s = known;
     }
   }
   __syncthreads();
-  const int start = start_s, mine = static_cast<int>(counts[e]), stop = start + (mine + pad - 1) / pad * pad;
+  const bool past = e == E;  // the block of the refused jobs and of the rows past the last expert's
+  const int start = start_s, mine = past ? J - known_s : static_cast<int>(counts[e]);
+  const int stop = past ? n_rows : start + (mine + pad - 1) / pad * pad;
   if (tid == 0) {
-    krange[2 * e] = start / 64;
-    krange[2 * e + 1] = stop / 64;
+    if (!past) {
+      krange[2 * e] = start / 64;
+      krange[2 * e + 1] = stop / 64;
+    } else if (mine > 0) {
+      atomicCAS(status, 0, pd::kBadExpert);
+      *static_cast<volatile int*>(refused) = 1;
+    }
   }
-  for (int i = start / 128 + tid; i < stop / 128; i += kLayoutThreads) bgroup[i] = e;
+  for (int i = start / 128 + tid; i < stop / 128; i += kLayoutThreads) bgroup[i] = past ? -1 : e;
   for (int i = start + mine + tid; i < stop; i += kLayoutThreads) inv[i] = -1;
-  if (e == E - 1) {  // rows past the last expert's
-    for (int i = end_s / 128 + tid; i < n_rows / 128; i += kLayoutThreads) bgroup[i] = -1;
-    for (int i = end_s + tid; i < n_rows; i += kLayoutThreads) inv[i] = -1;
-  }
+  auto own = [&](long long x) { return past ? x < 0 || x >= E : x == e; };
   // a warp takes kPer * 32 consecutive jobs a round, so that kPer loads are in flight and a barrier serves 8192 jobs
   constexpr int kPer = 8, kRound = kPer * kLayoutThreads;
   int base = start;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kLayoutThreads) job_layout_kernel(const long l
     unsigned ball[kPer];
     int in_warp = 0;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) ball[i] = __ballot_sync(0xffffffffu, j + 32 * i < J && expert[j + 32 * i] == e);
+    for (int i = 0; i < kPer; ++i) ball[i] = __ballot_sync(0xffffffffu, j + 32 * i < J && own(expert[j + 32 * i]));
 #pragma unroll
     for (int i = 0; i < kPer; ++i) in_warp += __popc(ball[i]);
     if (lane == 0) warp_sum_s[turn][warp] = in_warp;
@@ -1065,11 +1065,13 @@ extern "C" int pd_rowscale(const void* x, const float* s, void* y, long long row
   return PD_CHECK_LAUNCH();
 }
 extern "C" int pd_job_layout(const long long* expert, int J, int E, int pad, int n_rows, long long* pos, int* inv,
-                             int* bgroup, int* krange, long long* counts, int* status, void* stream) {
+                             int* bgroup, int* krange, long long* counts, int* status, int* refused, void* stream) {
   if (J <= 0 || E <= 0 || E > 8192 || (pad != 128 && pad != 256) || n_rows % 128 != 0) return 5;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  job_count_kernel<<<E, kLayoutThreads, 0, st>>>(expert, J, E, counts, pos, status);
-  job_layout_kernel<<<E, kLayoutThreads, 0, st>>>(expert, J, E, pad, n_rows, counts, pos, inv, bgroup, krange);
+  if (status == nullptr || refused == nullptr) return 5;
+  job_count_kernel<<<E, kLayoutThreads, 0, st>>>(expert, J, counts);
+  job_layout_kernel<<<E + 1, kLayoutThreads, 0, st>>>(expert, J, E, pad, n_rows, counts, pos, inv, bgroup, krange, status,
+                                                      refused);
   return PD_CHECK_LAUNCH();
 }
 extern "C" int pd_job_rowmap(const int* inv, void* rowmap, int n_rows, int k, int c, void* stream) {

@@ -102,7 +102,8 @@ def rows_combine(padded: Tensor, pos: Tensor, w: Tensor | None, tokens: int, k: 
 
 def job_layout(expert: Tensor, n_experts: int, pad: int, n_rows: int) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
     """`(pos [J], inv [n_rows], bgroup [n_rows / 128], krange [E, 2], counts [E])` of the jobs `expert [J]` (int64)
-    sorted stably by expert, every expert's run padded to a multiple of `pad` rows. Two launches."""
+    sorted stably by expert, every expert's run padded to a multiple of `pad` rows. Two launches. A job whose expert lies
+    outside `[0, n_experts)` is refused: `nv.raise_refused` raises from the next routed call on, `nv.check_status` at once."""
     assert expert.dtype == torch.int64 and expert.is_contiguous() and expert.dim() == 1
     dev, J = expert.device, expert.numel()
     i32 = torch.empty(n_rows + n_rows // 128 + 2 * n_experts, dtype=torch.int32, device=dev)
@@ -110,10 +111,10 @@ def job_layout(expert: Tensor, n_experts: int, pad: int, n_rows: int) -> tuple[T
     i64 = torch.empty(J + n_experts, dtype=torch.int64, device=dev)
     pos, counts = i64.split([J, n_experts])
     lib = _lib()
-    lib.pd_job_layout.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int] + [C.c_void_p] * 7
+    lib.pd_job_layout.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int] + [C.c_void_p] * 8
     _check(lib.pd_job_layout(expert.data_ptr(), J, n_experts, pad, n_rows, pos.data_ptr(), inv.data_ptr(),
                              bgroup.data_ptr(), krange.data_ptr(), counts.data_ptr(),
-                             nv.status_word().data_ptr(), _s()), "job_layout")
+                             nv.status_word().data_ptr(), nv.refused_ptr(), _s()), "job_layout")
     nv.count_launch()
     return pos, inv, bgroup, krange.view(n_experts, 2), counts
 

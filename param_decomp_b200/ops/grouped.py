@@ -84,6 +84,7 @@ class JobLayout:
 
     @classmethod
     def build(cls, expert_of_job: Tensor, n_experts: int) -> "JobLayout":
+        _raise_refused(expert_of_job)
         J = expert_of_job.numel()
         # static upper bound on rows so shapes do not depend on the routing (no host sync)
         n_rows = (J + n_experts * (PAD - 1) + PAD - 1) // PAD * PAD
@@ -138,6 +139,7 @@ class JobLayout:
     def combine(self, padded: Tensor, route_w: Tensor) -> Tensor:
         """`y[n] = sum_s route_w[n, s] * padded[row of job (n, s)]`: job rows back to tokens with the
         routing weights applied. `route_w [N, k]`."""
+        _raise_refused(padded)
         N, k = route_w.shape
         if _fast_rows(padded):
             return _RowsToTokens.apply(padded, route_w.float().contiguous(), self)
@@ -151,6 +153,11 @@ class JobLayout:
     def gather_rows(self, padded: Tensor) -> Tensor:
         """Padded sorted rows -> job order."""
         return _GatherRows.apply(padded, self.pos, self.n_rows, self)
+
+
+def _raise_refused(t: Tensor) -> None:
+    if t.is_cuda:
+        nv.raise_refused()
 
 
 def _fast_rows(t: Tensor) -> bool:
@@ -295,6 +302,7 @@ def grouped_site(x: Tensor, V: Tensor, U: Tensor, W: Tensor | None, layout: JobL
                  delta: Tensor | None, route: Tensor | None, grad_V: Tensor | None, grad_U: Tensor | None,
                  need_wgrad: bool) -> Tensor:
     """All arguments already in padded sorted-job order (`layout.scatter_rows`)."""
+    _raise_refused(x)
     rowscale = d_eff = None
     if route is not None:
         rowscale = route.float()
@@ -308,6 +316,7 @@ def grouped_site(x: Tensor, V: Tensor, U: Tensor, W: Tensor | None, layout: JobL
 
 def grouped_linear(x: Tensor, W: Tensor, layout: JobLayout) -> Tensor:
     """Frozen expert bank `y_j = x_j W[e(j)]^T` (clean forward)."""
+    _raise_refused(x)
     y = torch.empty(x.shape[0], W.shape[1], device=x.device, dtype=torch.bfloat16)
     nv.gemm(x.contiguous(), W, y, bgroup_of_mblock=layout.bgroup, cta_group=PAIR)
     return y
@@ -360,6 +369,7 @@ class _GroupedLinearTrainable(torch.autograd.Function):
 
 def grouped_linear_trainable(x: Tensor, W: Tensor, b: Tensor | None, layout: JobLayout) -> Tensor:
     """Per-expert trainable linear on padded sorted job rows (`layout.scatter_rows`)."""
+    _raise_refused(x)
     return _GroupedLinearTrainable.apply(x, W, b, layout)
 
 
@@ -423,6 +433,7 @@ def grouped_site_mapped(x: Tensor, V: Tensor, U: Tensor, W: Tensor, layout: JobL
                         seed: int, stream: int, row_offset: int, delta: Tensor | None, route: Tensor | None, k: int,
                         grad_V: Tensor | None, grad_U: Tensor | None, need_wgrad: bool) -> Tensor:
     """`x` padded job rows; `ci [N, k c]` bf16 in token order; `delta`, `route [N]` per token."""
+    _raise_refused(x)
     c = V.shape[-1]
     rowmap = layout.rowmap(k, c)
     rowscale = d_tok = None

@@ -119,14 +119,42 @@ def _status_ptr(device_index: int) -> int:
     return _status_word(device_index).data_ptr()
 
 
+@lru_cache(maxsize=8)
+def _refused_word(device_index: int) -> tuple[torch.Tensor, C.c_int]:
+    word = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+    return word, C.c_int.from_address(word.data_ptr())
+
+
+def refused_ptr() -> int:
+    """Pinned host int32 a kernel sets beside the status word when it refuses its input, readable without a wait."""
+    return _refused_word(torch._C._cuda_getDevice())[0].data_ptr()
+
+
+def raise_refused() -> None:
+    """Raise if a kernel that has run on this device refused its input (costs a host read; the calls that take routed
+    jobs make it, so an error reaches a caller that never looks at the status word, one call late at worst)."""
+    if _refused_word(torch._C._cuda_getDevice())[1].value != 0:
+        check_status()
+
+
+def status_message(code: int) -> str:
+    """What a status code says (`pd::StatusCode`)."""
+    if code == 6:
+        return "a routed job named an expert outside the bank (status code 6)"
+    return f"a device-side wait timed out (status code {code})"
+
+
+def clear_status() -> None:
+    status_word().zero_()
+    _refused_word(torch._C._cuda_getDevice())[1].value = 0
+
+
 def check_status() -> None:
     """Synchronising check of the status word; raises if a bounded wait ran out or a kernel refused its input."""
     code = int(status_word().item())
     if code != 0:
-        status_word().zero_()
-        if code == 6:
-            raise NativeError("a routed job named an expert outside the bank")
-        raise NativeError(f"a device-side wait timed out (status code {code})")
+        clear_status()
+        raise NativeError(status_message(code))
 
 
 _STEP_SEED: tuple[int, int] | None = None  # (seed64 of the running step, device address of the word holding it)

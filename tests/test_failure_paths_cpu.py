@@ -179,3 +179,10 @@ def test_a_rank_that_raises_between_steps_ends_the_others_quickly():
         assert not any(alive), "a rank was still waiting for its dead peer"
         assert out[1][0].startswith("RuntimeError: the data source of rank 1 failed")
         assert out[0][0] != "finished" and out[0][1] < 120, out[0]
+
+
+def test_status_codes_say_what_happened():
+    from param_decomp_b200.ops import native
+
+    assert "expert outside the bank" in native.status_message(6) and "timed out" not in native.status_message(6)
+    assert all("timed out" in native.status_message(code) for code in (1, 2, 3, 4))

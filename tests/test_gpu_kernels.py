@@ -1139,3 +1139,32 @@ def test_delta_rule_vanishing_decay(nv, dk, dv):
         for i in range(B):  # sequence 0 holds the vanishing decays
             err = float((a[i].double() - b[i]).norm() / (b[i].norm() + 1e-9))
             assert err < 3e-6, (name, i, err)
+
+
+def test_job_layout_refuses_unknown_experts(nv):
+    """Jobs of experts that do not exist: reported through the status word and to the next routed call, rows of their own
+    outside every expert's blocks, everybody else's layout as without them."""
+    from param_decomp_b200.ops.grouped import JobLayout
+
+    E = 7
+    e = torch.randint(0, E, (9000,), generator=torch.Generator().manual_seed(0))
+    bad = torch.tensor([0, 17, 1500, 8191, 8192, 8999])
+    e[bad] = torch.tensor([-1, E, 2**40, -(2**40), E + 1, -7])
+    good = torch.ones(9000, dtype=torch.bool)
+    good[bad] = False
+    a, b = JobLayout.build(e.cuda(), E), JobLayout.build(e[good], E)
+    torch.cuda.synchronize()
+    pos, blocks = a.pos.cpu(), b.bgroup.numel()
+    assert torch.equal(pos[good], b.pos) and pos.unique().numel() == 9000
+    assert torch.equal(a.inv.cpu()[pos], torch.arange(9000, dtype=torch.int32)) and int((a.inv >= 0).sum()) == 9000
+    assert torch.equal(a.krange.cpu(), b.krange) and torch.equal(a.counts.cpu(), b.counts)
+    owner = torch.nn.functional.pad(b.bgroup, (0, max(0, a.bgroup.numel() - blocks)), value=-1)[: a.bgroup.numel()]
+    assert torch.equal(a.bgroup.cpu(), owner) and bool((a.bgroup.cpu()[pos[bad] >> 7] == -1).all())
+    with pytest.raises(nv.NativeError, match="expert"):
+        JobLayout.build(e[good].cuda(), E)
+    nv.check_status()  # reported once
+    JobLayout.build(e.cuda(), E)
+    with pytest.raises(nv.NativeError, match="expert"):
+        nv.check_status()
+    JobLayout.build(e[good].cuda(), E)
+    _done(nv)
