@@ -1361,16 +1361,17 @@ struct PdGemmCall {
 // 11.1 / 10.2 / 8.9 / 12.5 (64 takes two waves); 4096 x 768 x 768 11.4 / 10.4 / 13.6 / 16.7; 4096 x 768 x 8192
 // 46.6 / 55.2 / 86 / 123: a single CTA re-reads more per K block, which a long K loop pays for (27.2 against 28.1 at
 // K = 4096). Mask products 4096 x 512 x 768: 14.9 / 15.3 / 11.4; a wider mask product stays on pairs.
+// A call may ask for a width; 64 columns serve plain and faithfulness products on one CTA that own their matrices, every
+// other call that asks for them gets 256.
 static void choose_tile(const PdGemmCall& c, int& bn, int& single_cta) {
-  bn = c.bn == 128 || c.bn == 64 ? c.bn : 256;
+  const bool mask = c.epi == EPI_MASK_FWD || c.epi == EPI_MASK_BWD;
+  const bool own = c.bgroup_of_mblock == nullptr && c.kblock_range == nullptr && c.ag_world <= 1 && c.rs_world <= 1;
+  bn = c.bn == 128 || (c.bn == 64 && own && !mask && c.cta_group != 2) ? c.bn : 256;
   single_cta = c.cta_group == 1;
-  if (c.bn != 0 || c.cta_group != 0 || c.max_ctas != 0 || c.bgroup_of_mblock != nullptr || c.kblock_range != nullptr ||
-      c.ag_world > 1 || c.rs_world > 1)
-    return;
+  if (c.bn != 0 || c.cta_group != 0 || c.max_ctas != 0 || !own) return;
   constexpr long long kSms = 148;
   const long long rows = static_cast<long long>((c.M + BM - 1) / BM) * c.batch * (c.split_k > 1 ? c.split_k : 1);
   auto one_wave = [&](int n) { return rows * ((c.N + n - 1) / n) <= kSms; };
-  const bool mask = c.epi == EPI_MASK_FWD || c.epi == EPI_MASK_BWD;
   if (!mask && one_wave(64))
     bn = 64;
   else if (one_wave(128))
@@ -1384,7 +1385,6 @@ extern "C" int pd_gemm(const PdGemmCall* c, void* stream_v) {
   if (c->M <= 0 || c->N <= 0 || c->batch <= 0 || c->K0 <= 0) return kBadArgument;
   if (c->epi != EPI_PLAIN && (c->batch != 1 || c->accumulate || c->out_fp32)) return kBadArgument;
   if (c->accumulate && !c->out_fp32) return kBadArgument;
-  if (c->bn == 64 && c->epi != EPI_PLAIN && c->epi != EPI_FAITH) return kBadArgument;
   const int nout = (c->epi == EPI_MASK_FWD && c->out1 != nullptr) ? 2 : 1;
   int bn, single_cta;
   choose_tile(*c, bn, single_cta);

@@ -1168,3 +1168,20 @@ def test_job_layout_refuses_unknown_experts(nv):
         nv.check_status()
     JobLayout.build(e[good].cuda(), E)
     _done(nv)
+
+
+def test_gemm_width_requests_that_do_not_apply(nv):
+    """A mask product or a CTA pair asked for with 64 columns runs at 256: same bits as that request."""
+    torch.manual_seed(0)
+    M, N, K = 640, 392, 136
+    a, b = torch.randn(M, K, device="cuda").to(bf), torch.randn(N, K, device="cuda").to(bf)
+    ci, delta = torch.rand(M, N, device="cuda").to(bf), torch.rand(M, device="cuda")
+    res = []
+    for bn in (64, 256):
+        A, H, y = (torch.zeros(M, N, device="cuda", dtype=bf) for _ in range(3))
+        nv.gemm(a, b, A, epi=nv.EPI_MASK_FWD, out1=H, ci=ci, delta=delta, seed=3, rng_stream=1, bn=bn)
+        nv.gemm(a, b, y, bn=bn, cta_group=2)
+        res.append((A, H, y))
+    _done(nv)
+    assert all(torch.equal(p, q) for p, q in zip(*res))
+    assert rel(res[0][2], a.float() @ b.float().T) < 2**-8
