@@ -88,9 +88,11 @@ class JobLayout:
         J = expert_of_job.numel()
         # static upper bound on rows so shapes do not depend on the routing (no host sync)
         n_rows = (J + n_experts * (PAD - 1) + PAD - 1) // PAD * PAD
-        # Two kernels while their blocks (one per expert, each walking all jobs) are short: at 2^19 jobs a walk is 64
-        # rounds of 8192 jobs; longer lists take the sort below.
-        if expert_of_job.is_cuda and 0 < J <= 1 << 19 and n_experts <= 8192 and expert_of_job.dtype == torch.int64:
+        # Two kernels whose blocks (one per expert) each walk all jobs, or the sort below, about 40 kernels. Kernels / sort on
+        # the device, us: 65,536 jobs and 42 experts 29 / 158, 1024 experts 113 / 154, 2048 217 / 154; 2^19 jobs and 256
+        # experts 233 / 254, 512 425 / 225; 2^18 and 512 218 / 186; 8192 jobs and 4096 experts 107 / 174, 8192 266 / 173.
+        short = n_experts <= 256 or (n_experts <= 4096 and n_experts * J <= 1 << 26)
+        if expert_of_job.is_cuda and 0 < J <= 1 << 19 and short and expert_of_job.dtype == torch.int64:
             pos, inv, bgroup, krange, counts = ew.job_layout(expert_of_job.contiguous(), n_experts, PAD, n_rows)
             return cls(pos, n_rows, bgroup, krange, counts, inv)
         # (a scatter-add, not bincount: bincount sizes its output from the data and synchronises)

@@ -1185,3 +1185,17 @@ def test_gemm_width_requests_that_do_not_apply(nv):
     _done(nv)
     assert all(torch.equal(p, q) for p, q in zip(*res))
     assert rel(res[0][2], a.float() @ b.float().T) < 2**-8
+
+
+@pytest.mark.parametrize("J,E,kernels", [(1 << 14, 4096, True), ((1 << 14) + 1, 4096, False), (100, 4097, False),
+                                         (1 << 19, 256, True), (1 << 18, 257, False), ((1 << 19) + 1, 2, False)])
+def test_job_layout_rule_by_size(nv, J, E, kernels):
+    """Both sides of each line of the choice between the kernels and the sort give the same layout."""
+    from param_decomp_b200.ops.grouped import JobLayout
+
+    e = torch.randint(0, E, (J,), generator=torch.Generator().manual_seed(E))
+    a, b = JobLayout.build(e.cuda(), E), JobLayout.build(e, E)
+    assert (a.inv is not None) == kernels
+    for f in ("pos", "bgroup", "krange", "counts"):
+        assert torch.equal(getattr(a, f).cpu(), getattr(b, f)), f
+    _done(nv)
