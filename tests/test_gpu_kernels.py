@@ -1199,3 +1199,13 @@ def test_job_layout_rule_by_size(nv, J, E, kernels):
     for f in ("pos", "bgroup", "krange", "counts"):
         assert torch.equal(getattr(a, f).cpu(), getattr(b, f)), f
     _done(nv)
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (5, 8), (33, 24), (70, 128), (9, 136), (3, 1024), (200, 14336), (37, 2056)])
+def test_rowscale_narrow_and_wide_rows(nv, rows, d):
+    from param_decomp_b200.ops import elementwise as ew
+
+    x, s = torch.randn(rows, d, device="cuda").to(bf), torch.rand(rows, device="cuda")
+    y = ew.rowscale(x, s)
+    _done(nv)
+    assert torch.equal(y, (x.float() * s[:, None]).to(bf))
