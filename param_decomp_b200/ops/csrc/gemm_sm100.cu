@@ -656,28 +656,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
       }
       __syncwarp();
       constexpr int nboxes = BN / 32, kWarpsPerRow = kEpiWarps<NOUT> / 4;
-      auto tile_is_real = [&](long long t) {
-        if (!args.bgroup_of_mblock) return true;
-        int b2, mb2, nb2, sp2;
-        decode(t, b2, mb2, nb2, sp2);
-        return args.bgroup_of_mblock[mb2] >= 0;
-      };
-      auto next_real_tile = [&](long long t) {
-        while (t < num_tiles && !tile_is_real(t)) t += tstride;
-        return t;
-      };
       // first unit of this warp at or after tile t (a warp may own no column of a narrow tail tile)
       auto first_unit_from = [&](long long t) {
-        t = next_real_tile(t);
         while (t < num_tiles) {
           int b2, mb2, nb2, sp2;
           decode(t, b2, mb2, nb2, sp2);
           if (nb2 * BN + grp * 32 < args.N) break;
-          t = next_real_tile(t + tstride);
+          t += tstride;
         }
         return t;
       };
-      // Called by the whole warp (coordinates in uniform registers); one elected lane issues. `after_stores`:
+      // Called by the whole warp (coordinates in uniform registers); lane 0 issues. `after_stores`:
       // first wait until the TMA stores that still read the destination slot have finished reading.
       auto issue_load = [&](long long t, int j, int slot, bool after_stores) {
         int b2 = 0, mb2 = 0, nb2 = 0, sp2 = 0;
@@ -702,7 +691,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         issue_load(t0u, grp, 0, false);
       }
       bool failed = false;
-      for (long long t = next_real_tile(tile0); t < num_tiles && !failed; t = next_real_tile(t + tstride)) {
+      for (long long t = tile0; t < num_tiles && !failed; t += tstride) {
         int b, mb, nb, sp;
         decode(t, b, mb, nb, sp);
         int kb_lo_e, kb_hi_e;
