@@ -11,7 +11,8 @@
 //     S = Q K_n^T  (TMEM, two buffers)  ->  online softmax in registers  ->  P_n (bf16, TMEM)  ->  O += P_n V_n (TMEM)
 // S of the next 64 keys is formed while the softmax warps work on the current ones, also across items, so they wait
 // neither for the tensor pipe nor for a new item's first loads. A row's scores are read once into registers; P goes
-// back to tensor memory over the scores it came from, as the A operand of P V, and never touches shared memory. O
+// back to tensor memory over the scores it came from, as the A operand of P V, and never touches shared memory (steps of
+// published kernels: the online softmax of FlashAttention, P in tensor memory as in CUTLASS's Blackwell attention example). O
 // stays in TMEM; a warp rescales its rows there when the maximum of one has grown. The exponents always refer to the
 // running maximum: with an older one as reference (rescaling only past a growth of 2^8) a row's largest probability is a
 // rounded number instead of exactly 1 and the error against 64 bits is 1.5 to 3% larger (forward 93 and 173 us so, 99 and
