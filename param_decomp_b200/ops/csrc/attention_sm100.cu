@@ -18,7 +18,8 @@
 // rounded number instead of exactly 1 and the error against 64 bits is 1.5 to 3% larger (forward 93 and 173 us so, 99 and
 // 198 us as it is). Tiles off the diagonal of
 // unsegmented calls take no mask arithmetic. 256 TMEM columns and at most 98 KB a CTA; K and V halves share one ring in the
-// order the tensor pipe takes them. What bounds it is the exponentials (16 lanes a clock: 1024 cycles per 128 x 128).
+// order the tensor pipe takes them. What bounds it is a warp's chain of load, maximum, exponentials and
+// store per step: tensor pipe 26 / 51% (width 64 / 128), exponentials 39 / 41%, issue slots 43 / 48% busy.
 // B 64, T 512, 12 heads of 64: 99 us (152 us with one 128-key S at a time, P through shared memory and O in registers);
 // B 4, T 2048, 32 / 8 heads of 128: 198 us, 695 TFLOP/s (440 us).
 //
@@ -35,7 +36,8 @@
 // reductions are one contiguous 512-byte run; a last pass casts it to bf16 rows. The pass over dO and O that forms D
 // also clears that scratch. With one warpgroup that took every step in turn and 16-byte atomics at row pitch, B 64,
 // T 512, 12 heads of 64 took 420 us and B 4, T 2048, 32 / 8 heads of 128 995 us (D, scratch and cast included);
-// now 285 and 570 us. What is left is the chain S -> P -> dP -> dS -> dQ of a tile: 512 columns hold one tile.
+// now 289 and 580 us. What is left is the chain S -> P -> dP -> dS -> dQ of a tile, of which 512 columns hold one: tensor
+// pipe 25 / 49% busy, every other unit less.
 //
 // Every wait is bounded; on a time-out the status word is set and all roles leave.
 //

@@ -7,6 +7,7 @@
 // (the state forward, its cotangent backward) give each column to four lanes of a warp, 32 columns to a block and
 // DV / 32 blocks to a (batch, head): 64 heads of 128 x 128 then make 1024 warps instead of 256, and a token costs a
 // warp one pass over 32 registers and two shuffles. k, q and the block's values arrive 16 tokens at a time by cp.async.
+// Bound by the chain of a token (two warps a scheduler, issue slots 36% busy) and the shared-memory pipe (61 - 65%).
 //
 // What else the backward needs - dq, dk, dg, dbeta - are sums over columns. They leave the serial chain: within a
 // 64-token chunk they are products of [64, 64], [64, DK] and [64, DV] tiles with the chunk's boundary states, one block
@@ -15,7 +16,7 @@
 //
 // Forward + backward, B 4, T 512, H 16, 128 x 128: 7.62 ms with one thread per column, the state of every token
 // written out and read back in the backward, and two passes over shared memory per token;
-// 0.74 ms now, errors against 64 bits 1.1e-7 .. 2.6e-7 (1.5e-7 .. 3.2e-7 before).
+// 0.76 ms so, errors against 64 bits 1.1e-7 .. 2.6e-7 (1.5e-7 .. 3.2e-7 before).
 //
 // Replaces the XLA einsum + scan lowering of param_decomp/target_ports/qwen3_5_moe.py:89-158,187-293;
 // the torch restatement of the same recurrence (`models/ports.py`) is the oracle.
@@ -243,8 +244,9 @@ __global__ void __launch_bounds__(kSerialThreads) delta_bwd_state_kernel(
 // Decays are differences of a running sum of g kept in 64 bits (in 32 its rounding would show in D), as are the
 // exponentials and the few hundred final additions of dg. A g below -10^4 enters the sum as -10^4: exp of either is 0 in
 // 32 bits, but with -inf the differences past it would be NaN and with -10^18 the later terms of the sum would be lost.
-// 256 threads, a thread owns 4 tokens x DK / 16 columns of dq, dk. Bound by the fp32 FMA rate: 7.3 M FMA per chunk at
-// 128 x 128; the operand tiles take 222 KB of shared memory, one block per SM.
+// 256 threads, a thread owns 4 tokens x DK / 16 columns of dq, dk. 7.3 M FMA per chunk at 128 x 128; the
+// operand tiles take 217 KB of shared memory, one block per SM. Two warps a scheduler at 222 registers leave latency bare:
+// FMA pipe 35%, shared-memory pipe 39%, issue slots 29% busy.
 constexpr int kGradThreads = 256;
 constexpr float kMinLogDecay = -1.0e4f;
 __device__ __forceinline__ double log_decay(float g) { return g < kMinLogDecay ? kMinLogDecay : g; }

@@ -47,9 +47,9 @@ constexpr int BM = 128;
 constexpr int BK = 64;
 // Epilogue warps: two per TMEM lane quarter; four in the TMA-fed mask form, whose arithmetic (about 16 instructions an
 // element, chains of seven Philox rounds) two warps per scheduler issue at a quarter of the rate. 32768 x 768 -> 4096
-// components: mask gradient 306 -> 281 us; the forward stays at 262 us, with or without the Philox draw (259): its
-// operand loads and box traffic share L2 with 0.8 GB of results, 1085 cycles a K block against 512 for the MMAs. One slot
-// per warp and five pipeline stages instead of two and three: 281 / 307 us.
+// components: mask gradient 306 -> 281 us; the forward stays at 262 us, with or without the Philox draw (259), 1085 cycles
+// a K block against 512 for the MMAs: tensor pipe 43%, issue slots 46%, DRAM 36%, L2 32% busy, the epilogue's dependent
+// steps in between. One slot per warp and five pipeline stages instead of two and three: 281 / 307 us.
 template <int NOUT>
 constexpr int kEpiWarps = NOUT == 4 ? 16 : 8;
 template <int NOUT>
